@@ -40,11 +40,12 @@ struct lu_handle_s {
   int num_sms = 148;
   // workspace (device)
   DevStatus* st = nullptr;
+  // the panel leaves' packets, then the counters: one allocation, cleared
+  // together before each factorisation
+  ulonglong2* leaf_pkt = nullptr;
   unsigned* counters = nullptr;
   int n_counters = 0;
   int next_counter = 0;
-  lub::LeafScratch<double> leaf64{};
-  lub::LeafScratch<float> leaf32{};
   lub::PivotList plist{};      // pivot lists of the trailing stream
   lub::PivotList plistP{};     // pivot lists of the panel stream (look-ahead)
   cudaStream_t sP = nullptr;   // high-priority panel stream (look-ahead)
@@ -54,7 +55,7 @@ struct lu_handle_s {
   // columns first, the rest after the panel has started (LU_B200_LA_SPLIT)
   int la_split = 1;  // mixed look-ahead: the next panel's columns first, then the rest
   // leaf tuning: recursion leaf width and CTA cap, without / with look-ahead
-  int leaf_w64 = 32, leaf_w32 = 64, leaf_ctas = 148;
+  int leaf_w64 = 32, leaf_w32 = 32, leaf_ctas = 148;
   int leaf_w64_la = 16, leaf_w32_la = 32, leaf_ctas_la = 48;
   // low-precision trailing update: CTAs of the persistent kernel (0: one CTA
   // per tile); under look-ahead the update beside a running panel leaves
@@ -206,9 +207,15 @@ struct lu_handle_s {
     cudaFree(p);
     allocs.erase(std::remove(allocs.begin(), allocs.end(), p), allocs.end());
   }
+  size_t clear_bytes() const { return sizeof(ulonglong2) * lub::kLeafPackets + sizeof(unsigned) * n_counters; }
   unsigned* take_counter() {
     if (next_counter >= n_counters) return nullptr;
     return counters + next_counter++;
+  }
+  // tag base of one leaf's packets, distinct within a factorisation (0: none left)
+  unsigned take_leaf_tag() {
+    if (next_counter >= n_counters) return 0;
+    return 64u * (unsigned)++next_counter;
   }
 };
 

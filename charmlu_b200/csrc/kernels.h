@@ -22,27 +22,26 @@ int launch_gemm_f64_sub(const CUtensorMap& mapA, const CUtensorMap& mapB, const 
 int launch_gemm_f32_sub(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc, int M,
                         int N, int K, cudaStream_t s);
 
-// ---- unblocked panel leaf (cooperative, rows resident in shared memory)
-template <typename T>
-struct LeafScratch {
-  T* cand_val;     // [2][kMaxLeafCTAs]
-  int* cand_row;   // [2][kMaxLeafCTAs]
-  T* cand_data;    // [2][kMaxLeafCTAs][kMaxLeafW]
-  T* rowj;         // [2][kMaxLeafW]
-};
+// ---- unblocked panel leaf (rows resident in registers)
 constexpr int kMaxLeafCTAs = 160;
-constexpr int kMaxLeafW = 64;
+constexpr int kMaxLeafW = 64;         // tournament leaf's scratch
+constexpr int kLeafRowPackets = 22;   // 16-byte packets of a candidate row: 3 words each, at most 64 words
+constexpr int kLeafPackets = 2 * kMaxLeafCTAs * (1 + kLeafRowPackets);
+// widest leaf (32, 16 or 8) that num_sms CTAs hold for M rows
 template <typename T>
-int leaf_init();
-// Factor P[0:M, 0:ncols] (row-major, P = diagonal of the first column) with
-// partial pivoting; ipiv[j] = row_base + local pivot row.  Each swap is also
-// applied to the enclosing panel's other columns: prow0 points at the
-// panel's first column in the leaf's top row, the panel is pw wide and the
-// leaf starts lc0 columns in (prow0 = null: the leaf is the panel).
+int leaf_max_width(int M, int num_sms);
+// Factor P[0:M, 0:ncols] (row-major, P = diagonal of the first column, ncols
+// <= 32) with partial pivoting; ipiv[j] = row_base + local pivot row.  Its
+// interchanges are also applied to the enclosing panel's other columns:
+// prow0 points at the panel's first column in the leaf's top row, the panel
+// is pw wide and the leaf starts lc0 columns in (prow0 = null: the leaf is the
+// panel).  pkt: kLeafPackets packets zeroed before the first leaf that uses them;
+// each leaf since then has its own tag0, a multiple of 64 below 2^32.  alone:
+// no other kernel holds SMs beside this one (the leaf may be one cluster).
 template <typename T>
-int launch_getf2_leaf(T* P, int64_t lda, int M, int ncols, int32_t* ipiv, int row_base, const LeafScratch<T>& scr,
-                      unsigned* bar, DevStatus* st, int info_base, double thr, long long spin, int max_ctas,
-                      cudaStream_t s, T* prow0 = nullptr, int pw = 0, int lc0 = 0);
+int launch_getf2_leaf(T* P, int64_t lda, int M, int ncols, int32_t* ipiv, int row_base, ulonglong2* pkt,
+                      unsigned tag0, DevStatus* st, int info_base, double thr, long long spin, int max_ctas,
+                      bool alone, cudaStream_t s, T* prow0 = nullptr, int pw = 0, int lc0 = 0);
 
 // ---- tournament-pivoting leaf of the FP32 panels (tslu.cu)
 struct TsluScratch {

@@ -67,8 +67,6 @@ int ensure_kernels_init() {
   return once_per_device(g_init, [] {
     int s = gemm_f64_init();
     if (s == LU_OK) s = gemm_bf16_init();
-    if (s == LU_OK) s = leaf_init<double>();
-    if (s == LU_OK) s = leaf_init<float>();
     if (s == LU_OK) s = tslu_init();
     return s;
   });
@@ -140,13 +138,13 @@ int trsm64(Ctx64& c, const MatF64& Lm, int r0, int w, const MatF64& Bm, int rb, 
 // panel's columns, so the recursion needs no separate laswp
 int panel64(Ctx64& c, int c0, int w, int p0, int pw) {
   const int M = c.n - c0;
-  if (w <= c.leaf_w) {
-    unsigned* bar = c.h->take_counter();
-    if (!bar) return LU_ERR_NOMEM;
+  if (w <= std::min(c.leaf_w, leaf_max_width<double>(M, c.h->num_sms))) {
+    const unsigned tag = c.h->take_leaf_tag();
+    if (!tag) return LU_ERR_NOMEM;
     Prof pf(c.h, c.s, LU_PH_PANEL, (double)M * w * w);
-    return launch_getf2_leaf<double>(c.A.at(c0, c0), c.A.ld, M, w, c.ipiv + c0, c.base + c0, c.h->leaf64, bar,
-                                     c.h->st, c.base + c0, c.thr, c.h->spin, c.leaf_ctas, c.s, c.A.at(c0, p0), pw,
-                                     c0 - p0);
+    return launch_getf2_leaf<double>(c.A.at(c0, c0), c.A.ld, M, w, c.ipiv + c0, c.base + c0, c.h->leaf_pkt, tag,
+                                     c.h->st, c.base + c0, c.thr, c.h->spin, c.leaf_ctas, !c.h->cfg.lookahead, c.s,
+                                     c.A.at(c0, p0), pw, c0 - p0);
   }
   const int w1 = split_w(w), w2 = w - w1;
   LUB_TRY(panel64(c, c0, w1, p0, pw));
@@ -180,7 +178,7 @@ int factor_f64_schedule(lu_handle h, double* dA, int64_t lda, int32_t* ipiv, dou
   c.leaf_ctas = la ? h->leaf_ctas_la : h->leaf_ctas;
   LUB_TRY(c.A.init(dA, n, n, lda));
   LUB_CUDA(cudaMemsetAsync(h->st, 0, sizeof(DevStatus), s));
-  LUB_CUDA(cudaMemsetAsync(h->counters, 0, sizeof(unsigned) * h->n_counters, s));
+  LUB_CUDA(cudaMemsetAsync(h->leaf_pkt, 0, h->clear_bytes(), s));
   h->next_counter = 0;
   LUB_TRY(launch_iota(h->perm, n, s));
   if (!la) {
@@ -267,10 +265,7 @@ size_t lu_workspace_bytes(const lu_config* cfg) {
   size_t b = 0;
   b += sizeof(DevStatus);
   b += sizeof(unsigned) * (n / 2 + 1024);
-  b += 2 * kMaxLeafCTAs * (sizeof(double) + sizeof(int)) + 2 * kMaxLeafCTAs * kMaxLeafW * sizeof(double) +
-       2 * kMaxLeafW * sizeof(double);
-  b += 2 * kMaxLeafCTAs * (sizeof(float) + sizeof(int)) + 2 * kMaxLeafCTAs * kMaxLeafW * sizeof(float) +
-       2 * kMaxLeafW * sizeof(float);
+  b += sizeof(ulonglong2) * kLeafPackets;
   b += 2 * sizeof(int32_t) * (4 * kMaxBatch + 1);
   b += sizeof(int32_t) * 2 * n;
   b += sizeof(int) * (n / 64 + 2) + sizeof(unsigned);
@@ -300,15 +295,8 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
   // trailing-update tile counter (panels are >= 64 columns wide)
   h->n_counters = (int)(n / 2 + n / 64 + 1024);
   if (s == LU_OK) s = h->alloc(&h->st, 1);
-  if (s == LU_OK) s = h->alloc(&h->counters, h->n_counters);
-  if (s == LU_OK) s = h->alloc(&h->leaf64.cand_val, 2 * kMaxLeafCTAs);
-  if (s == LU_OK) s = h->alloc(&h->leaf64.cand_row, 2 * kMaxLeafCTAs);
-  if (s == LU_OK) s = h->alloc(&h->leaf64.cand_data, 2 * kMaxLeafCTAs * kMaxLeafW);
-  if (s == LU_OK) s = h->alloc(&h->leaf64.rowj, 2 * kMaxLeafW);
-  if (s == LU_OK) s = h->alloc(&h->leaf32.cand_val, 2 * kMaxLeafCTAs);
-  if (s == LU_OK) s = h->alloc(&h->leaf32.cand_row, 2 * kMaxLeafCTAs);
-  if (s == LU_OK) s = h->alloc(&h->leaf32.cand_data, 2 * kMaxLeafCTAs * kMaxLeafW);
-  if (s == LU_OK) s = h->alloc(&h->leaf32.rowj, 2 * kMaxLeafW);
+  if (s == LU_OK) s = h->alloc(&h->leaf_pkt, kLeafPackets + (h->n_counters + 3) / 4);
+  h->counters = reinterpret_cast<unsigned*>(h->leaf_pkt + kLeafPackets);
   if (s == LU_OK) s = h->alloc(&h->plist.dst, 2 * kMaxBatch);
   if (s == LU_OK) s = h->alloc(&h->plist.src, 2 * kMaxBatch);
   if (s == LU_OK) s = h->alloc(&h->plist.m, 1);
@@ -335,8 +323,8 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
   if (const char* e = getenv("LU_B200_LEAF_CTAS_LA")) h->leaf_ctas_la = std::max(1, atoi(e));
   if (const char* e = getenv("LU_B200_LEAF_W64")) h->leaf_w64 = std::min(32, std::max(2, atoi(e)));
   if (const char* e = getenv("LU_B200_LEAF_W64_LA")) h->leaf_w64_la = std::min(32, std::max(2, atoi(e)));
-  if (const char* e = getenv("LU_B200_LEAF_W32")) h->leaf_w32 = std::min(64, std::max(4, atoi(e)));
-  if (const char* e = getenv("LU_B200_LEAF_W32_LA")) h->leaf_w32_la = std::min(64, std::max(4, atoi(e)));
+  if (const char* e = getenv("LU_B200_LEAF_W32")) h->leaf_w32 = std::min(32, std::max(4, atoi(e)));
+  if (const char* e = getenv("LU_B200_LEAF_W32_LA")) h->leaf_w32_la = std::min(32, std::max(4, atoi(e)));
   if (const char* e = getenv("LU_B200_GEMM_CTAS")) h->gemm_ctas = std::max(0, atoi(e));
   if (const char* e = getenv("LU_B200_GEMM_RESERVE")) h->gemm_reserve = std::max(0, atoi(e));
   if (const char* e = getenv("LU_B200_GEMM_HELPER")) h->gemm_helper = atoi(e) != 0;
@@ -660,7 +648,7 @@ int lu_panel_factor(lu_handle h, double* dP, int64_t ldp, int64_t m, int32_t w, 
   c.base = (int)base;
   LUB_TRY(c.A.init(dP, m, w, ldp));
   // one barrier counter per leaf, from a pool cleared for this panel
-  LUB_CUDA(cudaMemsetAsync(h->counters, 0, sizeof(unsigned) * h->n_counters, s));
+  LUB_CUDA(cudaMemsetAsync(h->leaf_pkt, 0, h->clear_bytes(), s));
   h->next_counter = 0;
   return panel64(c, 0, w, 0, w);
 }

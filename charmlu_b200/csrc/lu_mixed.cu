@@ -180,18 +180,18 @@ int panel_gemm_tc(Ctx32& c, int r0, int M, int kc, int K, int n0, int N, int cen
 // the leaves swap rows across the whole panel (no laswp in the recursion)
 int panel32(Ctx32& c, int c0, int w, int p0, int pw) {
   const int M = c.n - c0;
-  if (w <= c.leaf_w) {
+  if (w <= std::min(c.leaf_w, leaf_max_width<float>(M, c.h->num_sms))) {
     Prof pf(c.h, c.s, LU_PH_PANEL, (double)M * w * w);
     if (c.h->tslu && c.h->tslu_scr.cand_idx) {
       const int rc = launch_tslu_leaf(c.A + (int64_t)c0 * c.ld + c0, c.ld, M, w, c.ipiv + c0, c0, c.h->tslu_scr,
                                       c.h->st, c0, c.thr, c.leaf_ctas, c.s, c.A + (int64_t)c0 * c.ld + p0, pw, c0 - p0);
       if (rc != LU_ERR_UNSUPPORTED) return rc;
     }
-    unsigned* bar = c.h->take_counter();
-    if (!bar) return LU_ERR_NOMEM;
-    return launch_getf2_leaf<float>(c.A + (int64_t)c0 * c.ld + c0, c.ld, M, w, c.ipiv + c0, c0, c.h->leaf32, bar,
-                                    c.h->st, c0, c.thr, c.h->spin, c.leaf_ctas, c.s, c.A + (int64_t)c0 * c.ld + p0,
-                                    pw, c0 - p0);
+    const unsigned tag = c.h->take_leaf_tag();
+    if (!tag) return LU_ERR_NOMEM;
+    return launch_getf2_leaf<float>(c.A + (int64_t)c0 * c.ld + c0, c.ld, M, w, c.ipiv + c0, c0, c.h->leaf_pkt, tag,
+                                    c.h->st, c0, c.thr, c.h->spin, c.leaf_ctas, !c.h->cfg.lookahead, c.s,
+                                    c.A + (int64_t)c0 * c.ld + p0, pw, c0 - p0);
   }
   const int w1 = split_w32(w), w2 = w - w1;
   LUB_TRY(panel32(c, c0, w1, p0, pw));
@@ -360,7 +360,7 @@ int factor_mixed(lu_handle h, cudaStream_t s, const double* rest_src, int64_t re
   CUtensorMap mapC;
   LUB_TRY(encode_tmap_2d(&mapC, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->A32, n, n, h->ld32 * 4, 32, 128,
                          CU_TENSOR_MAP_SWIZZLE_128B));
-  LUB_CUDA(cudaMemsetAsync(h->counters, 0, sizeof(unsigned) * h->n_counters, s));
+  LUB_CUDA(cudaMemsetAsync(h->leaf_pkt, 0, h->clear_bytes(), s));
   h->next_counter = 0;
   LUB_TRY(launch_iota(h->perm, n, s));
   if (!la) {
