@@ -45,11 +45,13 @@
 // Measured on B200, per column: FP64 order 2048 (cluster) 4.7 -> 1.5 us, FP32
 // order 10000 (cluster) 5.0 -> 1.5 us, FP32 order 65536 beside the trailing
 // update (48-CTA grid) 7.6 -> 4.3 us, against a leaf that kept its rows in
-// shared memory and took a grid barrier per column.  About 180 instructions
+// shared memory and took a grid barrier per column; one CTA of 256 rows alone
+// 1.1 us (FP64), 0.8 us (FP32).  About 180 instructions
 // per warp and column remain, most of them waiting on the one before.
 #pragma once
 #include <climits>
 
+#include "argmax.cuh"
 #include "common.cuh"
 #include "kernels.h"
 
@@ -60,38 +62,6 @@ constexpr int NT = 256;       // threads per CTA: 255 registers each, 8 warps to
 constexpr int NW = NT / 32;
 constexpr int kMaxCluster = 16;
 enum { kSingle = 0, kGrid = 1, kCluster = 2 };
-
-// Lane whose (a, pos) is best: largest a among lanes with ok, the lowest
-// position on ties; -1 when no lane is ok.  a >= 0 and not NaN where ok, so
-// its bit pattern orders as the value does.
-__device__ __forceinline__ int lowest_pos(unsigned mask, int pos) {
-  if (mask & (mask - 1u)) {
-    const int lane = threadIdx.x & 31;
-    const bool in = (mask >> lane) & 1u;
-    const unsigned best = __reduce_min_sync(0xffffffffu, in ? (unsigned)pos : 0xffffffffu);
-    mask = __ballot_sync(0xffffffffu, in && (unsigned)pos == best);
-  }
-  return __ffs((int)mask) - 1;
-}
-__device__ __forceinline__ int warp_best(float a, bool ok, int pos) {
-  const unsigned k = ok ? __float_as_uint(a) : 0u;
-  const unsigned m = __reduce_max_sync(0xffffffffu, k);
-  return lowest_pos(__ballot_sync(0xffffffffu, ok && k == m), pos);
-}
-__device__ __forceinline__ int warp_best(double a, bool ok, int pos) {
-  const unsigned hi = ok ? (unsigned)__double2hiint(a) : 0u;
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  bool in = ok && hi == mh;
-  unsigned mask = __ballot_sync(0xffffffffu, in);
-  if (mask & (mask - 1u)) {
-    const unsigned lo = in ? (unsigned)__double2loint(a) : 0u;
-    const unsigned ml = __reduce_max_sync(0xffffffffu, lo);
-    in = in && lo == ml;
-    mask = __ballot_sync(0xffffffffu, in);
-    return lowest_pos(mask, pos);
-  }
-  return __ffs((int)mask) - 1;
-}
 
 // Candidate (value, position) as a header's three words, and back
 __device__ __forceinline__ void key_words(float v, unsigned& a, unsigned& b) { a = __float_as_uint(v); b = 0; }
@@ -425,7 +395,9 @@ __global__ void __launch_bounds__(NT, 1) getf2_leaf_kernel(T* P, T* prow0, LeafA
     for (int u = 0; u < RPT; u++) {
       if (pos[u] == pj) pos[u] = ~j;
       else if (pos[u] == j) pos[u] = pj;
-      const T l = none ? v[u][0] : v[u][0] / piv;
+      // rows that are done or absent divide the pivot by itself: a zero
+      // numerator leaves the division's fast path, and its warp with it
+      const T l = none ? v[u][0] : (pos[u] >= 0 ? v[u][0] : piv) / piv;
       lbuf[j * LP + u * NT + tid] = l;
       m[u] = none ? T(0) : l;
     }
