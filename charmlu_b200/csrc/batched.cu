@@ -12,18 +12,20 @@
 // fill the tail (longest-processing-time-first balance).
 //
 // Per system (one CTA):
-//   n <= small threshold  the whole matrix and b in shared memory, unblocked
-//   otherwise             blocked right-looking LU in global memory (L2):
-//                         an m x nb panel factored in shared memory, its
-//                         swaps applied to the other columns and to b, the
-//                         U row by forward substitution, the trailing update
-//                         in 64 x 128 tiles with 4 x 4 register blocks per
-//                         thread, the tiles' C and L blocks double-buffered
-//                         in shared memory by async copies
+//   n <= small threshold  the whole matrix in shared memory (factor_small)
+//   otherwise             two-level blocked LU in global memory (factor_system)
 //   then                  blocked forward / backward substitution
-// On B200 the FP64 SIMT pipe has the same peak as FP64 DMMA, and these
-// per-SM problems are too small for the tensor-core tiles, so FP64 here runs
-// on the FP64 SIMT pipe.
+// What bounds it: an SM works on one system, phase after phase, so every
+// phase's latency counts as much as its arithmetic.  Panels keep their rows in
+// registers and rename rows instead of moving them (panel_regs); a panel of an
+// outer block is brought up to date as it is loaded; interchanges, U rows and
+// trailing update of an outer block go over the matrix together.
+// B200, 4096 systems of order 32 .. 1024 (log-uniform): FP64 64.5 -> 41.4 ms,
+// FP32 with refinement 71.9 -> 39.4 ms; one system of order 1024 on every SM:
+// FP64 14.3 -> 9.4 ms (trailing update 4.6, panels 1.2 + 0.9 for loading and
+// storing them, U rows of the outer blocks 1.0, substitution 0.8).  Results are
+// bit for bit those of the right-looking form with plain fmas that it
+// replaced: every element sees the same fmas and sums in the same order.
 //
 // LU_PREC_FP32: the FP32 copy of each matrix (workspace) is factored, then
 // FP64 refinement (r = b - A x against the FP64 A, FP32 correction solve,
@@ -31,8 +33,10 @@
 // steps.  One step is not enough at these orders: after one step r_hpl is
 // ~1e4 for a uniform n = 109 system (the remaining error lies along the
 // small singular directions); two steps bring it to O(1).
+#include <climits>
 #include <mutex>
 
+#include "argmax.cuh"
 #include "common.cuh"
 #include "kernels.h"
 
@@ -100,140 +104,6 @@ __device__ __forceinline__ void tuning_for(int n, int esize, int& nb, int& small
   }
 }
 
-template <typename T>
-__device__ __forceinline__ bool better(T v1, int r1, T v2, int r2) {
-  return r1 >= 0 && (r2 < 0 || v1 > v2 || (v1 == v2 && r1 < r2));
-}
-
-// block-wide argmax (value, row); lowest row on ties; -1 if no positive value.
-// One barrier: every warp reduces the NWARP per-warp candidates itself.  The
-// caller puts a barrier between the return and its next call (the slots are
-// reused).
-template <typename T>
-__device__ int block_argmax(T v, int r, T* sv, int* sr) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    T v2 = __shfl_xor_sync(0xffffffffu, v, o);
-    int r2 = __shfl_xor_sync(0xffffffffu, r, o);
-    if (better(v2, r2, v, r)) { v = v2; r = r2; }
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (lane == 0) { sv[warp] = v; sr[warp] = r; }
-  __syncthreads();
-  v = lane < NWARP ? sv[lane] : T(0);
-  r = lane < NWARP ? sr[lane] : -1;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    T v2 = __shfl_xor_sync(0xffffffffu, v, o);
-    int r2 = __shfl_xor_sync(0xffffffffu, r, o);
-    if (better(v2, r2, v, r)) { v = v2; r = r2; }
-  }
-  return r;
-}
-
-// Unblocked LU with partial pivoting of an m x w block in shared memory
-// (pitch ld), rows global row0.. ; pivots (local rows) into piv_s[w].
-// Columns beyond w are not touched.  Returns the 1-based first zero pivot.
-template <typename T>
-__device__ int getf2_smem(T* a, int ld, int m, int w, int* piv_s, T* sv, int* sr) {
-  int info = 0;
-  const int tid = threadIdx.x;
-  // candidate of column 0; later candidates come out of the update pass
-  T bv = 0;
-  int br = -1;
-  for (int i = tid; i < m; i += BT) {
-    const T v = fabs(a[i * ld]);
-    if (v > bv) { bv = v; br = i; }
-  }
-  for (int j = 0; j < w && j < m; j++) {
-    // its barrier also ends the previous update; the barrier after the
-    // swap separates this call from the next
-    int p = block_argmax(bv, br, sv, sr);
-    if (p < 0) {
-      p = j;
-      if (info == 0) info = j + 1;
-    }
-    if (tid == 0) piv_s[j] = p;
-    if (p != j)
-      for (int c = tid; c < w; c += BT) {
-        const T t = a[j * ld + c];
-        a[j * ld + c] = a[p * ld + c];
-        a[p * ld + c] = t;
-      }
-    __syncthreads();
-    // one pass per row: multiplier (true division), rank-1 update of the
-    // rest of the block, and the candidate of column j + 1
-    const T piv = a[j * ld + j];
-    const bool do_scale = piv != T(0) && !isnan(piv);
-    bv = 0;
-    br = -1;
-    for (int i = j + 1 + tid; i < m; i += BT) {
-      T* ar = a + i * ld;
-      if (do_scale) {
-        const T l = ar[j] / piv;
-        ar[j] = l;
-        for (int c = j + 1; c < w; c++) ar[c] = fma(-l, a[j * ld + c], ar[c]);
-      }
-      if (j + 1 < w) {
-        const T v = fabs(ar[j + 1]);
-        if (v > bv) { bv = v; br = i; }
-      }
-    }
-  }
-  __syncthreads();
-  return info;
-}
-
-// Blocked forward (unit L) and backward (U) substitution in global memory,
-// 32-row blocks: a warp-parallel GEMV over the solved part, then one warp
-// substitutes inside the 32 x 32 diagonal block.
-template <typename T>
-__device__ void solve_global(const T* LU, int n, T* x, T* s_acc) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int I0 = 0; I0 < n; I0 += 32) {
-    const int rows = min(32, n - I0);
-    for (int i = warp; i < rows; i += NWARP) {
-      const T* row = LU + (int64_t)(I0 + i) * n;
-      T acc = 0;
-      for (int j = lane; j < I0; j += 32) acc = fma(row[j], x[j], acc);
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) s_acc[i] = acc;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      T v = lane < rows ? x[I0 + lane] - s_acc[lane] : T(0);
-      for (int j = 0; j < rows; j++) {
-        const T xj = __shfl_sync(0xffffffffu, v, j);
-        if (lane > j && lane < rows) v = fma(-LU[(int64_t)(I0 + lane) * n + I0 + j], xj, v);
-      }
-      if (lane < rows) x[I0 + lane] = v;
-    }
-    __syncthreads();
-  }
-  const int nblk = (n + 31) / 32;
-  for (int bi = nblk - 1; bi >= 0; bi--) {
-    const int I0 = bi * 32, rows = min(32, n - I0), J0 = I0 + rows;
-    for (int i = warp; i < rows; i += NWARP) {
-      const T* row = LU + (int64_t)(I0 + i) * n;
-      T acc = 0;
-      for (int j = J0 + lane; j < n; j += 32) acc = fma(row[j], x[j], acc);
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (lane == 0) s_acc[i] = acc;
-    }
-    __syncthreads();
-    if (warp == 0) {
-      T v = lane < rows ? x[I0 + lane] - s_acc[lane] : T(0);
-      for (int j = rows - 1; j >= 0; j--) {
-        if (lane == j) v = v / LU[(int64_t)(I0 + j) * n + I0 + j];
-        const T xj = __shfl_sync(0xffffffffu, v, j);
-        if (lane < j) v = fma(-LU[(int64_t)(I0 + lane) * n + I0 + j], xj, v);
-      }
-      if (lane < rows) x[I0 + lane] = v;
-    }
-    __syncthreads();
-  }
-}
-
 // Element copy global -> shared through the async copy unit; pred false
 // zero-fills the destination (src-size 0: nothing is read).
 template <int BYTES>
@@ -246,395 +116,901 @@ __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async
 template <int N>
 __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Outer block width of the two-level blocking: the inner panels (nb
-// columns) update only the outer block's own columns and U rows; the rest of
+// Outer block width of the two-level blocking: the inner panels (nb columns)
+// are brought up to date inside the outer block as they come up; the rest of
 // the trailing matrix gets one update of depth kOuter per outer block.
 template <typename T>
 constexpr int outer_block() { return sizeof(T) == 8 ? 64 : 128; }
 
-// C[r0:r1, c0:c1] -= A[r0:r1, kk0:kk0+K] * A[kk0:kk0+K, c0:c1] (K <=
-// outer_block<T>(); the L and U blocks final in global memory) over TM x TN
-// tiles, a 4 x 4 block of outputs per thread: rows tr*4 .. +3, columns
-// tc + (TN/4) j (consecutive across the lanes of a column group: conflict-free
-// shared reads of U and coalesced global accesses; a warp spans 32*4/TN row
-// groups, whose L rows sit in distinct banks with the pitch K + 1).  Shapes:
-// 64 x 128 for the outer block's trailing update, 256 x 32 for the narrow
-// update of its own columns, 32 x 256 for its U rows.  Per column tile the U
-// slice is staged once; the row tiles' L blocks stream through two shared
-// buffers with the async copy unit.  Each thread's C values are loaded at
-// the start of its tile and subtracted after the products are summed, so
-// their latency hides behind the k loop.
-// smem (reusing the panel's space):  Ut [K][TN] | Lt[2] [TM][K+1]
-template <typename T, int TM, int TN>
-__device__ void update_block(T* A, int n, int r0, int r1, int c0, int c1, int kk0, int K, unsigned char* smem) {
-  static_assert((TM / 4) * (TN / 4) == BT, "one 4 x 4 block of outputs per thread");
-  constexpr int GX = TN / 4;
-  if (r0 >= r1 || c0 >= c1 || K <= 0) return;
-  const int tid = threadIdx.x, tr = tid / GX, tc = tid % GX;
-  const int KP = K + 1;
-  T* ut = reinterpret_cast<T*>(smem);
-  T* lt = ut + (size_t)K * TN;
-  const int nrt = (r1 - r0 + TM - 1) / TM;
-  auto issue = [&](int t, int buf) {
-    const int rt = r0 + t * TM;
-    T* ldst = lt + (size_t)buf * TM * KP;
-    for (int idx = tid; idx < TM * K; idx += BT) {
-      const int r = idx / K, p = idx - r * K;
-      const bool ok = rt + r < r1;
-      cp_async_elem<sizeof(T)>(ldst + r * KP + p, ok ? A + (int64_t)(rt + r) * n + kk0 + p : A, ok);
-    }
-    cp_async_commit_group();
-  };
-  for (int ct = c0; ct < c1; ct += TN) {
-    // U slice (K x TN): all of a thread's loads in flight together
-    for (int base = 0; base < K * TN; base += BT * 8) {
-      T v[8];
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int idx = base + tid + u * BT;
-        const int p = idx / TN, c = idx % TN;
-        v[u] = (idx < K * TN && ct + c < c1) ? A[(int64_t)(kk0 + p) * n + ct + c] : T(0);
-      }
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int idx = base + tid + u * BT;
-        if (idx < K * TN) ut[idx] = v[u];
-      }
-    }
-    issue(0, 0);
-    for (int t = 0; t < nrt; t++) {
-      const int buf = t & 1;
-      const int rbase = r0 + t * TM + tr * 4;
-      T cv[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const int r = rbase + i, c = ct + tc + GX * j;
-          cv[i][j] = (r < r1 && c < c1) ? A[(int64_t)r * n + c] : T(0);
-        }
-      if (t + 1 < nrt) {
-        issue(t + 1, buf ^ 1);
-        cp_async_wait_group<1>();
-      } else {
-        cp_async_wait_group<0>();
-      }
-      __syncthreads();  // L tile t (and, at t = 0, the U slice) in shared memory
-      const T* ls = lt + (size_t)buf * TM * KP + (size_t)tr * 4 * KP;
-      T acc[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = T(0);
-      for (int p = 0; p < K; p++) {
-        T av[4], bv[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) av[i] = ls[i * KP + p];
-#pragma unroll
-        for (int j = 0; j < 4; j++) bv[j] = ut[p * TN + tc + GX * j];
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-          for (int j = 0; j < 4; j++) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int r = rbase + i;
-        if (r >= r1) break;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const int c = ct + tc + GX * j;
-          if (c < c1) A[(int64_t)r * n + c] = cv[i][j] - acc[i][j];
-        }
-      }
-      __syncthreads();  // buffer `buf` (and the U slice after the last tile) free for reuse
-    }
-  }
+// Shared memory beside the dynamic part.  Row numbers of one system fit 16 bits.
+template <typename T>
+struct BShared {
+  T key[2][NWARP];
+  int pos[2][NWARP];
+  int mv_n;
+  int info;
+  unsigned short src[kBatchMaxN];   // panel: row that now stands at each position
+  unsigned short ob[kBatchMaxN];    // the same since the outer block began
+  unsigned short perm[kBatchMaxN];  // the same since the system began
+  unsigned short mv_dst[256], mv_src[256];
+  unsigned short to[256];           // outer block: where each row of its old top block stands
+  T acc[32];
+  alignas(16) T diag[32][33];
+};
+
+// mma.sync.m16n8k4.f64 is bit for bit the chain of four fmas in k order
+// (checked against the host's fma), so sums over it are those of a scalar loop
+__device__ __forceinline__ void dmma_k4(double (&c)[4], double a0, double a1, double b0) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a0), "d"(a1), "d"(b0));
 }
 
-// First q < np with key[q] == v, found by one warp (all lanes get it); -1 if none.
-__device__ __forceinline__ int warp_find(const int* key, int np, int v) {
-  const int lane = threadIdx.x & 31;
-  for (int base = 0; base < np; base += 32) {
-    const unsigned m = __ballot_sync(0xffffffffu, base + lane < np && key[base + lane] == v);
-    if (m) return base + __ffs(m) - 1;
+// LU with partial pivoting of an m x kw panel at lb (column c of row r at
+// lb[c * mp + r]), kw <= W, m <= RPT * BT: as the single-matrix leaf, each
+// thread holds RPT whole rows in registers and rotates them, an interchange
+// renames two rows, the CTA's candidate takes one barrier per column.  On
+// return lb holds the multipliers by original row, urow[j][i] = U(j, j + i),
+// sh.src[d] = the original row at position d.  Returns the 1-based first
+// column without a usable pivot (0: none).  rowbuf: [2][NWARP][W].
+template <typename T, int W, int RPT>
+__device__ __noinline__ int panel_regs(T* lb, int mp, int m, int kw, T* rowbuf, T* urow, T* zero, BShared<T>& sh) {
+  constexpr int V = 16 / (int)sizeof(T);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  T v[RPT][W];
+  int pos[RPT];
+#pragma unroll
+  for (int u = 0; u < RPT; u++) {
+    const int r = tid + u * BT;
+    pos[u] = r < m ? r : INT_MIN;
+#pragma unroll
+    for (int i = 0; i < W; i++) v[u][i] = (r < m && i < kw) ? lb[i * mp + r] : T(0);
   }
+  if (tid < W) zero[tid] = T(0);
+  int info = 0;
+  const int steps = min(kw, m);
+#pragma unroll 1
+  for (int j = 0; j < steps; j++) {
+    const int buf = j & 1;
+    T* rows = rowbuf + buf * NWARP * W;
+    {
+      T bv = 0;
+      int bp = -1, bu = 0;
+#pragma unroll
+      for (int u = 0; u < RPT; u++) {
+        const T x = fabs(v[u][0]);
+        if (pos[u] >= 0 && (x > bv || (x == bv && bp >= 0 && pos[u] < bp))) {
+          bv = x;
+          bp = pos[u];
+          bu = u;
+        }
+      }
+      const int wl = warp_best(bv, bp >= 0, bp);
+      if (lane == max(wl, 0)) {
+        sh.key[buf][warp] = bv;
+        sh.pos[buf][warp] = wl < 0 ? -1 : bp;
+#pragma unroll
+        for (int u = 0; u < RPT; u++)
+          if (RPT == 1 || bu == u) {
+#pragma unroll
+            for (int i = 0; i < W; i += V) {
+              int4 q;
+              memcpy(&q, &v[u][i], 16);
+              *reinterpret_cast<int4*>(&rows[warp * W + i]) = q;
+            }
+          }
+      }
+    }
+    __syncthreads();
+    const T ck = lane < NWARP ? sh.key[buf][lane] : T(0);
+    const int cp = lane < NWARP ? sh.pos[buf][lane] : -1;
+    const int cw = warp_best(ck, cp >= 0, cp);
+    const bool none = cw < 0;
+    const int p = none ? j : sh.pos[buf][max(cw, 0)];
+    const T* pr = none ? zero : rows + max(cw, 0) * W;
+    if (none) {
+      if (info == 0) info = j + 1;
+#pragma unroll
+      for (int u = 0; u < RPT; u++)
+        if (pos[u] == j) {
+#pragma unroll
+          for (int i = 0; i < W; i++) urow[j * W + i] = v[u][i];
+        }
+    } else if (warp == (j & (NWARP - 1))) {
+      for (int k = lane; k < W; k += 32) urow[j * W + k] = pr[k];
+    }
+    const T piv = pr[0];
+    T mu[RPT];
+#pragma unroll
+    for (int u = 0; u < RPT; u++) {
+      if (pos[u] == p) pos[u] = ~j;
+      else if (pos[u] == j) pos[u] = p;
+      // rows that are done or absent divide the pivot by itself: a zero
+      // numerator leaves the division's fast path, and its warp with it
+      const T l = none ? v[u][0] : (pos[u] >= 0 ? v[u][0] : piv) / piv;
+      const int r = tid + u * BT;
+      if (r < m) lb[j * mp + r] = l;
+      mu[u] = none ? T(0) : l;
+    }
+#pragma unroll
+    for (int c = 0; c < W; c += V) {
+      T pv[V];
+      const int4 q = *reinterpret_cast<const int4*>(pr + c);
+      memcpy(pv, &q, 16);
+#pragma unroll
+      for (int e = 0; e < V; e++) {
+        if (c + e == 0) continue;
+#pragma unroll
+        for (int u = 0; u < RPT; u++) v[u][c + e - 1] = fma(-mu[u], pv[e], v[u][c + e]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < RPT; u++) v[u][W - 1] = T(0);
+  }
+#pragma unroll
+  for (int u = 0; u < RPT; u++)
+    if (pos[u] != INT_MIN) sh.src[pos[u] >= 0 ? pos[u] : ~pos[u]] = (unsigned short)(tid + u * BT);
+  __syncthreads();
+  return info;
+}
+
+template <typename T, int W>
+__device__ __forceinline__ int panel_any(T* lb, int mp, int m, int kw, T* rowbuf, T* urow, T* zero, BShared<T>& sh) {
+  if (m <= BT) return panel_regs<T, W, 1>(lb, mp, m, kw, rowbuf, urow, zero, sh);
+  if (m <= 2 * BT) return panel_regs<T, W, 2>(lb, mp, m, kw, rowbuf, urow, zero, sh);
+  if constexpr (W * sizeof(T) <= 128) {
+    if (m <= 3 * BT) return panel_regs<T, W, 3>(lb, mp, m, kw, rowbuf, urow, zero, sh);
+  }
+  if constexpr (W * sizeof(T) <= 64) return panel_regs<T, W, 4>(lb, mp, m, kw, rowbuf, urow, zero, sh);
   return -1;
 }
 
-// One warp: the interchanges (K0 + j) <-> piv[K0 + j], j = 0 .. S-1, in order,
-// composed into one simultaneous assignment row mdst[q] <- row msrc[q]
-// (q < the returned count, at most 2 S rows); pos / cont are scratch of 2 S.
-__device__ int compose_moves(const int* piv, int K0, int S, int* pos, int* cont, int* mdst, int* msrc) {
-  const int lane = threadIdx.x & 31;
-  int np = 0;
-  for (int j = 0; j < S; j++) {
-    const int a = K0 + j, b = piv[K0 + j];
-    if (a == b) continue;
-    int ia = warp_find(pos, np, a);
-    if (ia < 0) {
-      if (lane == 0) { pos[np] = a; cont[np] = a; }
-      ia = np++;
-      __syncwarp();
-    }
-    int ib = warp_find(pos, np, b);
-    if (ib < 0) {
-      if (lane == 0) { pos[np] = b; cont[np] = b; }
-      ib = np++;
-      __syncwarp();
-    }
-    if (lane == 0) {
-      const int t = cont[ia];
-      cont[ia] = cont[ib];
-      cont[ib] = t;
-    }
-    __syncwarp();
-  }
-  int mm = 0;
-  for (int base = 0; base < np; base += 32) {
-    const int q = base + lane;
-    const bool mv = q < np && pos[q] != cont[q];
-    const unsigned m = __ballot_sync(0xffffffffu, mv);
-    if (mv) {
-      const int o = mm + __popc(m & ((1u << lane) - 1u));
-      mdst[o] = pos[q];
-      msrc[o] = cont[q];
-    }
-    mm += __popc(m);
-  }
-  __syncwarp();
-  return mm;
+// Value of the factored panel at (position d, column c); W: urow's pitch
+template <typename T>
+__device__ __forceinline__ T panel_value(const T* lb, int mp, const T* urow, int W, const unsigned short* src, int d,
+                                         int c) {
+  return c < d ? lb[c * mp + src[d]] : urow[d * W + c - d];
 }
 
-// Row moves A[mdst[q], ca:cb] <- A[msrc[q], ca:cb] (q < mm <= 256), every
-// source read before any destination is written: 128-column chunks staged in
-// shared memory (buf, mm x 128 elements), 16 loads in flight per thread.
+// Positions whose row changed (map[d] != d, d < m) as moves mv_dst <- mv_src,
+// both offset by base; call between barriers, sh.mv_n = 0 before.
 template <typename T>
-__device__ void apply_moves(T* A, int n, const int* mdst, const int* msrc, int mm, int ca, int cb, T* buf) {
+__device__ __forceinline__ void list_moves(BShared<T>& sh, const unsigned short* map, int m, int base) {
+  for (int d = threadIdx.x; d < m; d += BT) {
+    const int s = map[d];
+    if (s != d) {
+      const int o = atomicAdd(&sh.mv_n, 1);
+      sh.mv_dst[o] = (unsigned short)(base + d);
+      sh.mv_src[o] = (unsigned short)(base + s);
+    }
+  }
+}
+
+// map <- map after the moves (rows base + ..): map[dst] = old map[src]
+template <typename T>
+__device__ __forceinline__ void compose_map(BShared<T>& sh, unsigned short* map, int base) {
   const int tid = threadIdx.x;
-  const int tot = mm * 128;
-  for (int c0 = ca; c0 < cb; c0 += 128) {
-    const int w = min(128, cb - c0);
-    for (int base = 0; base < tot; base += BT * 16) {
-      T v[16];
+  unsigned short t = 0;
+  if (tid < sh.mv_n) t = map[sh.mv_src[tid] - base];
+  __syncthreads();
+  if (tid < sh.mv_n) map[sh.mv_dst[tid] - base] = t;
+}
+
+// The listed row moves on columns [ca, cb) minus [xa, xb): per pass every
+// source of up to E x BT elements is read before any destination is written.
+// sr, sc: the strides of a row and of a column of A.
+template <typename T, int E>
+__device__ __forceinline__ void apply_moves(T* A, int64_t sr, int64_t sc, const BShared<T>& sh, int ca, int xa, int xb,
+                                            int cb) {
+  const int tid = threadIdx.x, mm = sh.mv_n;
+  const int nl = xa - ca, ncols = nl + cb - xb;
+  if (mm == 0 || ncols <= 0) return;
+  const int lg = 31 - __clz(max(1, E * BT / mm)), CW = 1 << lg;  // columns per pass, a power of two
+  for (int c0 = 0; c0 < ncols; c0 += CW) {
+    T v[E];
 #pragma unroll
-      for (int u = 0; u < 16; u++) {
-        const int idx = base + tid + u * BT;
-        const int q = idx >> 7, c = idx & 127;
-        v[u] = (idx < tot && c < w) ? A[(int64_t)msrc[q] * n + c0 + c] : T(0);
-      }
-#pragma unroll
-      for (int u = 0; u < 16; u++) {
-        const int idx = base + tid + u * BT;
-        if (idx < tot) buf[idx] = v[u];
-      }
+    for (int e = 0; e < E; e++) {
+      const int idx = tid + e * BT, q = idx >> lg, k = c0 + (idx & (CW - 1));
+      if (q < mm && k < ncols) v[e] = A[sh.mv_src[q] * sr + (k < nl ? ca + k : xb + k - nl) * sc];
     }
     __syncthreads();
-    for (int idx = tid; idx < tot; idx += BT) {
-      const int q = idx >> 7, c = idx & 127;
-      if (c < w) A[(int64_t)mdst[q] * n + c0 + c] = buf[idx];
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      const int idx = tid + e * BT, q = idx >> lg, k = c0 + (idx & (CW - 1));
+      if (q < mm && k < ncols) A[sh.mv_dst[q] * sr + (k < nl ? ca + k : xb + k - nl) * sc] = v[e];
+    }
+  }
+}
+
+// NB rows of one column (pitch up) by forward substitution, one fma per
+// element in k order, in registers
+template <typename T, int NB>
+__device__ __forceinline__ void solve_column(T* uc, int up, const T* lt, int lp) {
+  T u[NB];
+#pragma unroll
+  for (int i = 0; i < NB; i++) u[i] = uc[i * up];
+#pragma unroll
+  for (int p = 0; p < NB - 1; p++)
+#pragma unroll
+    for (int i = p + 1; i < NB; i++) u[i] = fma(-lt[i * lp + p], u[p], u[i]);
+#pragma unroll
+  for (int i = 1; i < NB; i++) uc[i * up] = u[i];
+}
+
+// U <- L^{-1} U by blocks of nb rows (4, 8, 16 or 32; Kp rows, a multiple of
+// nb; w <= CW columns; L unit lower at lt, pitch lp a multiple of 4; U at ut,
+// pitch up; all in shared memory): inside a block one thread per column; then
+// the rows below take the block's products summed from zero, four rows of a
+// column per thread.  Ends with a barrier.
+template <typename T, int CW>
+__device__ __forceinline__ void solve_rows(T* ut, int up, const T* lt, int lp, int Kp, int w, int nb) {
+  constexpr int V = 16 / (int)sizeof(T), RG = BT / CW;
+  const int tid = threadIdx.x, c = tid % CW, rg = tid / CW;
+  for (int q0 = 0; q0 < Kp; q0 += nb) {
+    if (rg == 0 && c < w) {
+      T* uc = ut + q0 * up + c;
+      const T* ld = lt + q0 * lp + q0;
+      if (nb == 32) solve_column<T, 32>(uc, up, ld, lp);
+      else if (nb == 16) solve_column<T, 16>(uc, up, ld, lp);
+      else if (nb == 8) solve_column<T, 8>(uc, up, ld, lp);
+      else solve_column<T, 4>(uc, up, ld, lp);
+    }
+    __syncthreads();
+    if (c < w) {
+      for (int i = q0 + nb + 4 * rg; i < Kp; i += 4 * RG) {  // Kp - q0 - nb is a multiple of 4
+        T acc[4] = {};
+        for (int p = 0; p < nb; p += V) {
+          T u[V], l[4][V];
+#pragma unroll
+          for (int e = 0; e < V; e++) u[e] = ut[(q0 + p + e) * up + c];
+#pragma unroll
+          for (int r = 0; r < 4; r++) {
+            const int4 q = *reinterpret_cast<const int4*>(&lt[(i + r) * lp + q0 + p]);
+            memcpy(l[r], &q, 16);
+#pragma unroll
+            for (int e = 0; e < V; e++) acc[r] = fma(l[r][e], u[e], acc[r]);
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++) ut[(i + r) * up + c] -= acc[r];
+      }
     }
     __syncthreads();
   }
 }
 
-// U rows: A[k0:k0+kw, c0:c1] <- L^{-1} A[k0:k0+kw, c0:c1], L the kw x kw
-// unit-lower block at lsm (pitch ld, shared memory); one column per thread.
+// m x kw block at (k0, k0) of A into lb (column c of row r at lb[c * mp + r])
 template <typename T>
-__device__ void u_rows(T* A, int n, int k0, int kw, int c0, int c1, const T* lsm, int ld) {
-  for (int c = c0 + threadIdx.x; c < c1; c += BT) {
-    T u[32];
+__device__ __forceinline__ void copy_panel(const T* A, int n, int k0, int kw, int m, T* lb, int mp) {
+  const int lg = kw > 1 ? 32 - __clz(kw - 1) : 0;
+  for (int idx = threadIdx.x; idx < (m << lg); idx += BT) {
+    const int r = idx >> lg, c = idx & ((1 << lg) - 1);
+    if (c < kw) cp_async_elem<sizeof(T)>(lb + c * mp + r, A + (int64_t)(k0 + r) * n + k0 + c, true);
+  }
+  cp_async_commit_group();
+  cp_async_wait_group<0>();
+}
+
+// Panel columns [k0, k0+kw), rows k0 .. k0+m, into lb, after the outer block's
+// earlier panels (columns K0 .. k0 of L, U rows at ut, pitch up): per nb of
+// them the products are summed from zero, then subtracted.
+__device__ __forceinline__ void load_panel(const double* A, int n, int k0, int kw, int m, int K0, int nb, double* lb,
+                                           int mp, const double* ut, int up) {
+  const int tid = threadIdx.x, Kp = k0 - K0;
+  if (Kp == 0) {
+    copy_panel(A, n, k0, kw, m, lb, mp);
+    return;
+  }
+  // one warp per 16 rows x 16 columns; columns 4 (j + 2 e) + t of a register,
+  // so a row's four lanes read 32 contiguous bytes
+  const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int nct = (kw + 15) / 16, nch = (m + 15) / 16;
+  for (int w = warp; w < nch * nct; w += NWARP) {
+    const int r = (w / nct) * 16 + g, cb = (w % nct) * 16;
+    const bool ok0 = r < m, ok1 = r + 8 < m;
+    const double* Ar = A + (int64_t)(k0 + r) * n;
+    const double* Ar8 = Ar + (int64_t)8 * n;
+    double cv[2][2][2];
 #pragma unroll
-    for (int i = 0; i < 32; i++) u[i] = i < kw ? A[(int64_t)(k0 + i) * n + c] : T(0);
+    for (int j = 0; j < 2; j++)
 #pragma unroll
-    for (int i = 1; i < 32; i++) {
-      if (i >= kw) break;
-#pragma unroll
-      for (int p = 0; p < 32; p++) {
-        if (p >= i) break;
-        u[i] = fma(-lsm[i * ld + p], u[p], u[i]);
+      for (int e = 0; e < 2; e++) {
+        const int c = cb + 4 * (j + 2 * e) + t;
+        cv[0][j][e] = (ok0 && c < kw) ? Ar[k0 + c] : 0.0;
+        cv[1][j][e] = (ok1 && c < kw) ? Ar8[k0 + c] : 0.0;
       }
+    const int bc = cb + (g >> 1) + 8 * (g & 1);  // column of this lane's B values (tile j: + 4 j)
+    for (int q = 0; q < Kp; q += nb) {
+      double acc[2][4] = {};
+      for (int kk = 0; kk < nb; kk += 16) {
+        double a0[4], a1[4];
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+          const int k = q + kk + 4 * s + t;
+          const bool in = kk + 4 * s < nb;
+          a0[s] = (in && ok0) ? Ar[K0 + k] : 0.0;
+          a1[s] = (in && ok1) ? Ar8[K0 + k] : 0.0;
+        }
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+          if (kk + 4 * s < nb) {
+            const double* ur = ut + (q + kk + 4 * s + t) * up;
+#pragma unroll
+            for (int j = 0; j < 2; j++) dmma_k4(acc[j], a0[s], a1[s], bc + 4 * j < kw ? ur[bc + 4 * j] : 0.0);
+          }
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+          for (int e = 0; e < 2; e++) cv[h][j][e] -= acc[j][2 * h + e];
     }
 #pragma unroll
-    for (int i = 0; i < 32; i++)
-      if (i < kw) A[(int64_t)(k0 + i) * n + c] = u[i];
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int c = cb + 4 * (j + 2 * e) + t;
+        if (c < kw) {
+          if (ok0) lb[c * mp + r] = cv[0][j][e];
+          if (ok1) lb[c * mp + r + 8] = cv[1][j][e];
+        }
+      }
+  }
+}
+__device__ __forceinline__ void load_panel(const float* A, int n, int k0, int kw, int m, int K0, int nb, float* lb,
+                                           int mp, const float* ut, int up) {
+  const int tid = threadIdx.x, Kp = k0 - K0;
+  copy_panel(A, n, k0, kw, m, lb, mp);
+  if (Kp == 0) return;
+  __syncthreads();
+  // 256 rows of L (nb columns) at a time through shared memory, one row and
+  // 16 of the panel's columns per thread, U broadcast
+  float* ls = lb + ((kw * mp + 3) & ~3);  // [256][33]
+  const int lg = 31 - __clz(nb), row = tid & 255, cb = (tid >> 8) * 16;
+  for (int q = 0; q < Kp; q += nb) {
+    for (int r0 = 0; r0 < m; r0 += 256) {
+      for (int idx = tid; idx < (256 << lg); idx += BT) {
+        const int i = idx >> lg, k = idx & (nb - 1);
+        if (r0 + i < m) cp_async_elem<4>(ls + i * 33 + k, A + (int64_t)(k0 + r0 + i) * n + K0 + q + k, true);
+      }
+      cp_async_commit_group();
+      cp_async_wait_group<0>();
+      __syncthreads();
+      if (r0 + row < m && cb < kw) {
+        float acc[16] = {};
+        for (int k = 0; k < nb; k++) {
+          const float l = ls[row * 33 + k];
+          const float* ur = ut + (q + k) * up + cb;
+          if (kw % 16 == 0) {
+#pragma unroll
+            for (int c = 0; c < 16; c += 4) {
+              const float4 b = *reinterpret_cast<const float4*>(ur + c);
+              acc[c] = fmaf(l, b.x, acc[c]);
+              acc[c + 1] = fmaf(l, b.y, acc[c + 1]);
+              acc[c + 2] = fmaf(l, b.z, acc[c + 2]);
+              acc[c + 3] = fmaf(l, b.w, acc[c + 3]);
+            }
+          } else {
+#pragma unroll
+            for (int c = 0; c < 16; c++)
+              if (cb + c < kw) acc[c] = fmaf(l, ur[c], acc[c]);
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 16; c++)
+          if (cb + c < kw) lb[(cb + c) * mp + r0 + row] -= acc[c];
+      }
+      __syncthreads();
+    }
   }
 }
 
-// Factor A (n x n row-major in global, ld = n) in place, recording the
-// pivots (global rows, LAPACK order) in piv; the caller permutes b.
+// Trailing update of one column tile: C[r0:r1, ct:ct+TN] -= L U over TM-row
+// tiles, L = A[.., kk0:kk0+K] streamed through two shared buffers of KS
+// columns, U at ut in shared memory (K = outer_block<T>()).  One barrier per
+// buffer; the copies of the next buffer and of the tile's own C values (each
+// thread's into its own slots of shared memory) land while the products are
+// summed (from zero, in k order), and C is prefetched into L2 two tiles ahead
+// (thousands of systems are far larger than L2).
+//
+// FP64: 64 x 128 tiles, a warp owns 32 x 16 outputs on dmma_k4, which computes
+// the transposed tile (A = U^T, B = L^T): the eight lanes of a fragment row
+// then lie along a row of C, so an access of C touches 4 lines of 64 bytes
+// instead of 8 of 32.  Both pitches are 4 mod 16 doubles: conflict-free
+// fragments.  The copies are issued between the products: in one go behind the
+// barrier they kept every warp from its products for a third of a tile (148
+// systems of order 1024, this update: 5.4 -> 4.6 ms, 2.7 of them the products
+// at the pipe's rate; 7.1 ms with 4 x 4 register blocks of plain fmas).
+//
+// FP32: 128 x 128 tiles, 8 rows x 4 columns per thread.  A warp's lanes share
+// the rows, so an L value is a broadcast and four of a row come in one 16-byte
+// load: 6 wavefronts per 32 fmas of a warp (2.7 ms at the same sizes; 3.1 with
+// the copies between the products).
 template <typename T>
-__device__ int factor_system(T* A, int n, int* piv, unsigned char* smem, T* sv, int* sr, int* piv_s) {
+struct Trail;
+template <>
+struct Trail<double> {
+  static constexpr int TM = 64, TN = 128, K = 64, KS = 64, UP = TN + 4, LP = KS + 4;
+};
+template <>
+struct Trail<float> {
+  static constexpr int TM = 128, TN = 128, K = 128, KS = 64, UP = TN, LP = KS + 4;
+};
+
+// Step t of the stream: columns (t % (K / KS)) KS .. of row tile t / (K / KS);
+// part p: BT elements of it
+template <typename T>
+__device__ __forceinline__ void stage_l_part(const T* A, int n, int r0, int r1, int kk0, int step, int p, T* lt) {
+  using C = Trail<T>;
+  constexpr int H = C::K / C::KS;
+  const int r = r0 + step / H * C::TM, k0 = kk0 + step % H * C::KS;
+  const int idx = threadIdx.x + p * BT, i = idx / C::KS, k = idx % C::KS;
+  const bool ok = r + i < r1;
+  cp_async_elem<sizeof(T)>(lt + (step & 1) * C::TM * C::LP + i * C::LP + k,
+                           ok ? A + (int64_t)(r + i) * n + k0 + k : A, ok);
+}
+template <typename T>
+__device__ __forceinline__ void stage_l(const T* A, int n, int r0, int r1, int kk0, int step, T* lt) {
+  using C = Trail<T>;
+#pragma unroll
+  for (int p = 0; p < C::TM * C::KS / BT; p++) stage_l_part(A, n, r0, r1, kk0, step, p, lt);
+  cp_async_commit_group();
+}
+
+// Rows [r, r + TM) of the column tile into L2
+template <typename T>
+__device__ __forceinline__ void prefetch_c(const T* A, int n, int r, int r1, int ct, int c1) {
+  using C = Trail<T>;
+  constexpr int LE = 128 / (int)sizeof(T), LPR = C::TN / LE;  // elements of a line, lines of a tile row
+  static_assert(C::TM * LPR == BT, "one line per thread");
+  const int i = r + threadIdx.x / LPR, j = ct + (threadIdx.x % LPR) * LE;
+  if (i < r1 && j < c1) asm volatile("prefetch.global.L2 [%0];" ::"l"(A + (int64_t)i * n + j));
+}
+constexpr int kAhead = 2;  // tiles between a prefetch and its use
+
+// lt: two L buffers, the first one's copies already committed; cs: BT slots of
+// TM TN / BT values
+__device__ __forceinline__ void trail_tile(double* A, int n, int r0, int r1, int ct, int c1, int kk0,
+                                           const double* ut, double* lt, double* cs) {
+  using C = Trail<double>;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int wr = (warp >> 3) * 32, wc = (warp & 7) * 16;
+  const int nrt = (r1 - r0 + C::TM - 1) / C::TM;
+  const int cb = ct + wc + g;  // columns cb, cb + 8
+  const bool okc[2] = {cb < c1, cb + 8 < c1};
+  cs += tid;
+  for (int tt = 0; tt < nrt; tt++) {
+    cp_async_wait_group<0>();
+    __syncthreads();  // L tile tt in shared memory; everyone is done with tile tt - 1
+    // rows rb + 8 i + e
+    const int rb = r0 + tt * C::TM + wr + 2 * t;
+    double* Cp = A + (int64_t)rb * n + cb;
+    prefetch_c(A, n, r0 + (tt + kAhead) * C::TM, r1, ct, c1);
+    const double* ls = lt + (tt & 1) * C::TM * C::LP + (wr + g) * C::LP + t;
+    const double* us = ut + t * C::UP + wc + g;
+    double acc[4][4] = {};
+#pragma unroll
+    for (int s = 0; s < C::K / 4; s++) {
+      const double u0 = us[4 * s * C::UP], u1 = us[4 * s * C::UP + 8];
+#pragma unroll
+      for (int i = 0; i < 4; i++) dmma_k4(acc[i], u0, u1, ls[8 * i * C::LP + 4 * s]);
+      if (s < 8) {
+        const int i = s >> 1, e = s & 1;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const bool ok = rb + 8 * i + e < r1 && okc[h];
+          cp_async_elem<8>(cs + (2 * s + h) * BT, ok ? Cp + (int64_t)(8 * i + e) * n + 8 * h : A, ok);
+        }
+        if (s == 7) cp_async_commit_group();
+      } else if (tt + 1 < nrt) {
+        stage_l_part(A, n, r0, r1, kk0, tt + 1, s - 8, lt);
+      }
+    }
+    cp_async_commit_group();
+    cp_async_wait_group<1>();
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int e = 0; e < 2; e++)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+          if (rb + 8 * i + e < r1 && okc[h])
+            Cp[(int64_t)(8 * i + e) * n + 8 * h] = cs[(4 * i + 2 * e + h) * BT] - acc[i][2 * h + e];
+  }
+}
+
+__device__ __forceinline__ void trail_tile(float* A, int n, int r0, int r1, int ct, int c1, int kk0, const float* ut,
+                                           float* lt, float* cs) {
+  using C = Trail<float>;
+  constexpr int H = C::K / C::KS;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wr = warp * 8;
+  const int nrt = (r1 - r0 + C::TM - 1) / C::TM;
+  cs += tid;
+  for (int tt = 0; tt < nrt; tt++) {
+    const int rb = r0 + tt * C::TM + wr, cb = ct + lane;  // columns cb + 32 j
+    float* Cp = A + (int64_t)rb * n + cb;
+    float acc[8][4] = {};
+#pragma unroll 1
+    for (int h = 0; h < H; h++) {
+      const int step = tt * H + h;
+      cp_async_wait_group<0>();
+      __syncthreads();  // L buffer of this step in shared memory; everyone is done with the step before
+      if (h == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const bool ok = rb + i < r1 && cb + 32 * j < c1;
+            cp_async_elem<4>(cs + (4 * i + j) * BT, ok ? Cp + (int64_t)i * n + 32 * j : A, ok);
+          }
+        prefetch_c(A, n, r0 + (tt + kAhead) * C::TM, r1, ct, c1);
+      }
+      if (step + 1 < nrt * H) stage_l(A, n, r0, r1, kk0, step + 1, lt);
+      const float* ls = lt + (step & 1) * C::TM * C::LP + wr * C::LP;
+      const float* us = ut + h * C::KS * C::UP + lane;
+#pragma unroll 2
+      for (int k = 0; k < C::KS; k += 4) {
+        float b[4][4];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) b[q][j] = us[(k + q) * C::UP + 32 * j];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const float4 l = *reinterpret_cast<const float4*>(ls + i * C::LP + k);
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            float v = acc[i][j];
+            v = fmaf(l.x, b[0][j], v);
+            v = fmaf(l.y, b[1][j], v);
+            v = fmaf(l.z, b[2][j], v);
+            v = fmaf(l.w, b[3][j], v);
+            acc[i][j] = v;
+          }
+        }
+      }
+    }
+    // C's copies were waited for with the last step's L buffer
+    static_assert(H >= 2, "");
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (rb + i < r1 && cb + 32 * j < c1) Cp[(int64_t)i * n + 32 * j] = cs[(4 * i + j) * BT] - acc[i][j];
+  }
+}
+
+// The outer block [K0, Kend) (Kend < n, Kend - K0 = outer_block<T>()) on the
+// columns right of it, one column tile at a time: its interchanges (sh.ob), its
+// U rows by solve_rows, the trailing update.
+template <typename T>
+__device__ __forceinline__ void outer_update(T* A, int n, int K0, int nb, unsigned char* smem, const BShared<T>& sh) {
+  using C = Trail<T>;
+  constexpr int K = C::K;
+  static_assert(K == outer_block<T>(), "");
+  const int tid = threadIdx.x, Kend = K0 + K;
+  T* ut = reinterpret_cast<T*>(smem);       // [K][UP]
+  T* lt = ut + K * C::UP;                   // [2][TM][LP]
+  T* cs = lt + 2 * C::TM * C::LP;           // [TM TN / BT][BT]
+  T* l11 = cs;                              // [K][K], until the U rows are solved
+  static_assert(C::TM * C::TN >= K * K, "");
+  static_assert((size_t)(K * C::UP + 2 * C::TM * C::LP + C::TM * C::TN) * sizeof(T) <= kBatchSmem, "");
+  for (int ct = Kend; ct < n; ct += C::TN) {
+    const int w = min(C::TN, n - ct), c = tid % C::TN, i0 = tid / C::TN;
+    constexpr int DI = BT / C::TN, E = K / DI;
+    // the pivot rows into ut, the old top rows into registers
+    T d[E];
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      const int i = i0 + e * DI;
+      cp_async_elem<sizeof(T)>(ut + i * C::UP + c, A + (int64_t)(K0 + sh.ob[i]) * n + ct + (c < w ? c : 0), c < w);
+    }
+    for (int idx = tid; idx < K * K; idx += BT)
+      cp_async_elem<sizeof(T)>(l11 + idx, A + (int64_t)(K0 + idx / K) * n + K0 + idx % K, true);
+    cp_async_commit_group();
+#pragma unroll
+    for (int e = 0; e < E; e++) d[e] = c < w ? A[(int64_t)(K0 + i0 + e * DI) * n + ct + c] : T(0);
+    cp_async_wait_group<0>();
+    __syncthreads();
+    stage_l(A, n, Kend, n, K0, 0, lt);  // lands while the U rows are solved, as do the first tiles of C
+    for (int tt = 0; tt < kAhead; tt++) prefetch_c(A, n, Kend + tt * C::TM, n, ct, n);
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      const int to = sh.to[i0 + e * DI];
+      if (to >= Kend && c < w) A[(int64_t)to * n + ct + c] = d[e];
+    }
+    solve_rows<T, C::TN>(ut, C::UP, l11, K, K, w, nb);
+#pragma unroll
+    for (int e = 0; e < E; e++)
+      if (c < w) A[(int64_t)(K0 + i0 + e * DI) * n + ct + c] = ut[(i0 + e * DI) * C::UP + c];
+    trail_tile(A, n, Kend, n, ct, n, K0, ut, lt, cs);
+    __syncthreads();  // ut, lt and cs free for the next column tile
+  }
+}
+
+// LU of an n x n system in shared memory (n <= the bucket's threshold):
+// a[c * mp + r], 16-column panels, everything right of a panel updated by one
+// fma per element and column in column order, as the unblocked elimination
+// does.  scr: rowbuf, urow and zero of panel_regs.
+template <typename T>
+__device__ int factor_small(T* A, int n, unsigned char* smem, BShared<T>& sh) {
+  constexpr int W = 16;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mp = n | 1;
+  T* a = reinterpret_cast<T*>(smem);
+  T* rowbuf = &sh.diag[0][0];  // 2 * NWARP * W + W * W + W <= 32 * 33 elements
+  T* urow = rowbuf + 2 * NWARP * W;
+  T* zero = urow + W * W;
+  static_assert(2 * NWARP * W + W * W + W <= 32 * 33, "");
+  for (int idx = tid; idx < n * n; idx += BT) a[(idx % n) * mp + idx / n] = A[idx];
+  int info = 0;
+  __syncthreads();
+  for (int k0 = 0; k0 < n; k0 += W) {
+    const int m = n - k0, kw = min(W, m), k1 = k0 + kw;
+    T* lb = a + k0 * mp + k0;
+    const int pi = panel_regs<T, W, 1>(lb, mp, m, kw, rowbuf, urow, zero, sh);
+    if (pi && !info) info = k0 + pi;
+    if (tid == 0) sh.mv_n = 0;
+    __syncthreads();
+    list_moves(sh, sh.src, m, k0);
+    __syncthreads();
+    apply_moves<T, 16>(a, 1, mp, sh, 0, k0, k1, n);
+    // the panel's own columns: rows of the top block, and the moved rows below
+    {
+      T v[2];
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int idx = tid + e * BT, d = idx / W, c = idx % W;  // top rows, then the list
+        v[e] = T(0);
+        if (d < W) {
+          if (d < kw && c < kw) v[e] = panel_value(lb, mp, urow, W, sh.src, d, c);
+        } else if (d - W < sh.mv_n && c < kw) {
+          v[e] = lb[c * mp + sh.mv_src[d - W] - k0];
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const int idx = tid + e * BT, d = idx / W, c = idx % W;
+        if (d < W) {
+          if (d < kw && c < kw) lb[c * mp + d] = v[e];
+        } else if (d - W < sh.mv_n && c < kw && sh.mv_dst[d - W] >= k1) {
+          lb[c * mp + sh.mv_dst[d - W] - k0] = v[e];
+        }
+      }
+    }
+    compose_map(sh, sh.perm, 0);
+    __syncthreads();
+    if (k1 >= n) break;
+    // U rows: one thread per column
+    if (k1 + tid < n) {
+      T* uc = a + (k1 + tid) * mp + k0;
+      T u[W];
+#pragma unroll
+      for (int i = 0; i < W; i++) u[i] = uc[i];
+#pragma unroll
+      for (int p = 0; p < W - 1; p++)
+#pragma unroll
+        for (int i = p + 1; i < W; i++) u[i] = fma(-lb[p * mp + i], u[p], u[i]);
+#pragma unroll
+      for (int i = 1; i < W; i++) uc[i] = u[i];
+    }
+    __syncthreads();
+    // the rest: two rows per lane, their multipliers in registers
+    const int rest = n - k1, nch = (rest + 63) / 64;
+    for (int w = warp; w < NWARP; w += NWARP) {
+      const int ch = w % nch, per = NWARP / nch;
+      if (w / nch >= per) break;
+      const int r0 = k1 + ch * 64 + lane, r1 = r0 + 32;
+      T l0[W], l1[W];
+#pragma unroll
+      for (int k = 0; k < W; k++) {
+        l0[k] = r0 < n ? a[(k0 + k) * mp + r0] : T(0);
+        l1[k] = r1 < n ? a[(k0 + k) * mp + r1] : T(0);
+      }
+      for (int c = k1 + w / nch; c < n; c += per) {
+        T* col = a + c * mp;
+        T v0 = r0 < n ? col[r0] : T(0), v1 = r1 < n ? col[r1] : T(0);
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+          const T u = col[k0 + k];
+          v0 = fma(-l0[k], u, v0);
+          v1 = fma(-l1[k], u, v1);
+        }
+        if (r0 < n) col[r0] = v0;
+        if (r1 < n) col[r1] = v1;
+      }
+    }
+    __syncthreads();
+  }
+  for (int idx = tid; idx < n * n; idx += BT) A[idx] = a[(idx % n) * mp + idx / n];
+  return info;
+}
+
+// Factor A (n x n row-major in global, ld = n) in place; sh.perm[i] = the
+// original row that ends at row i.  Returns the 1-based first column without
+// a usable pivot (0: none).
+//
+// Two-level blocking.  A panel of an outer block first gets the U rows of the
+// block's earlier panels for its own columns, then its rows are loaded through
+// the products with those panels, so inside the block no column is written
+// before its panel comes up; after the panel its interchanges are applied to
+// the block's other columns.  The columns left of the block take its composed
+// interchanges when it is done, those right of it in outer_update.
+template <typename T>
+__device__ int factor_system(T* A, int n, unsigned char* smem, BShared<T>& sh) {
   const int tid = threadIdx.x;
   int nb, small;
   tuning_for(n, (int)sizeof(T), nb, small);
-  if (n <= small) {
-    const int ld = n + 1;
-    T* a = reinterpret_cast<T*>(smem);
-    for (int idx = tid; idx < n * n; idx += BT) a[(idx / n) * ld + idx % n] = A[idx];
-    __syncthreads();
-    const int info = getf2_smem(a, ld, n, n, piv_s, sv, sr);
-    for (int j = tid; j < n; j += BT) piv[j] = piv_s[j];
-    for (int idx = tid; idx < n * n; idx += BT) A[idx] = a[(idx / n) * ld + idx % n];
-    __syncthreads();
-    return info;
-  }
+  for (int i = tid; i < n; i += BT) sh.perm[i] = (unsigned short)i;
+  if (n <= small) return factor_small<T>(A, n, smem, sh);
+  constexpr int NB = outer_block<T>();
+  T* ut = reinterpret_cast<T*>(smem);
   int info = 0;
-  const int ld = nb + 1;
-  T* panel = reinterpret_cast<T*>(smem);                  // n x (nb+1)
-  __shared__ int sw_dst[64], sw_src[64], sw_m;             // composed row moves of a panel
-  // an outer block's composed interchanges (at most 2 x outer_block rows)
-  __shared__ int s_pos[256], s_cont[256], s_mdst[256], s_msrc[256];
   for (int k0 = 0; k0 < n; k0 += nb) {
-    const int kw = min(nb, n - k0), m = n - k0;
-    // panel in: eight loads in flight per thread
-    for (int base = 0; base < m * kw; base += BT * 8) {
-      T v[8];
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int idx = base + tid + u * BT;
-        const int i = idx / kw, c = idx - i * kw;
-        v[u] = idx < m * kw ? A[(int64_t)(k0 + i) * n + k0 + c] : T(0);
+    const int kw = min(nb, n - k0), m = n - k0, mp = m | 1, c1 = k0 + kw;
+    const int K0 = k0 - k0 % NB, Kend = min(n, K0 + NB), Kp = k0 - K0;
+    const int up = sizeof(T) == 8 ? kw + 2 : kw;
+    const int W = kw <= 8 && sizeof(T) == 8 ? 8 : (kw <= 16 ? 16 : 32);
+    T* lb = ut + ((Kp * up + 3) & ~3);  // [kw][mp]
+    T* rowbuf = lb + ((kw * mp + 3) & ~3);
+    T* urow = rowbuf + 2 * NWARP * W;
+    T* zero = urow + W * W;
+    if (Kp == 0)
+      for (int i = tid; i < n - K0; i += BT) sh.ob[i] = (unsigned short)i;
+    if (Kp > 0) {
+      T* lt = lb;  // [Kp][Kp + 4], before the panel takes the space
+      const int lg = kw > 1 ? 32 - __clz(kw - 1) : 0;
+      for (int idx = tid; idx < (Kp << lg); idx += BT) {
+        const int i = idx >> lg, c = idx & ((1 << lg) - 1);
+        if (c < kw) ut[i * up + c] = A[(int64_t)(K0 + i) * n + k0 + c];
       }
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int idx = base + tid + u * BT;
-        const int i = idx / kw, c = idx - i * kw;
-        if (idx < m * kw) panel[i * ld + c] = v[u];
+      for (int idx = tid; idx < Kp * Kp; idx += BT) {
+        const int i = idx / Kp, k = idx - i * Kp;
+        lt[i * (Kp + 4) + k] = A[(int64_t)(K0 + i) * n + K0 + k];
+      }
+      __syncthreads();
+      solve_rows<T, 32>(ut, up, lt, Kp + 4, Kp, kw, nb);
+      for (int idx = tid; idx < (Kp << lg); idx += BT) {
+        const int i = idx >> lg, c = idx & ((1 << lg) - 1);
+        if (c < kw) A[(int64_t)(K0 + i) * n + k0 + c] = ut[i * up + c];
       }
     }
+    load_panel(A, n, k0, kw, m, K0, nb, lb, mp, ut, up);
     __syncthreads();
-    const int pi = getf2_smem(panel, ld, m, kw, piv_s, sv, sr);
+    int pi;
+    if (W == 8) {
+      if constexpr (sizeof(T) == 8) pi = panel_any<T, 8>(lb, mp, m, kw, rowbuf, urow, zero, sh);
+      else pi = 0;
+    } else if (W == 16) {
+      pi = panel_any<T, 16>(lb, mp, m, kw, rowbuf, urow, zero, sh);
+    } else {
+      pi = panel_any<T, 32>(lb, mp, m, kw, rowbuf, urow, zero, sh);
+    }
     if (pi && !info) info = k0 + pi;
-    for (int idx = tid; idx < m * kw; idx += BT) {
-      const int i = idx / kw, c = idx - i * kw;
-      A[(int64_t)(k0 + i) * n + k0 + c] = panel[i * ld + c];
-    }
-    // Two-level blocking.  Inside an outer block of NB columns each panel
-    // swaps rows, solves its U rows and updates all rows below only within
-    // the outer block's columns.  The columns left and right of the outer
-    // block are untouched until its last panel: then its interchanges,
-    // composed into one assignment of rows, are applied to them in one pass;
-    // its U rows right of it are solved (blocked forward substitution with its
-    // unit-lower L11); and the rest of the trailing matrix gets one update of
-    // depth NB.
-    constexpr int NB = outer_block<T>();
-    const int K0 = k0 - k0 % NB, Kend = min(n, K0 + NB);
-    const int c1 = k0 + kw;
-    // this panel's swaps (the pivot record, then one warp composes them into
-    // one assignment of the affected rows: row dst <- row src, at most 2 kw
-    // moves), applied to the outer block's other columns with every source
-    // read before any destination is written
-    for (int j = tid; j < kw; j += BT) piv[k0 + j] = k0 + piv_s[j];
-    __syncthreads();
-    if (tid < 32) {
-      const int mm = compose_moves(piv, k0, kw, s_pos, s_cont, sw_dst, sw_src);
-      if (tid == 0) sw_m = mm;
-    }
-    __syncthreads();
     {
-      // at most NB - kw <= 120 columns: four threads per column, each a
-      // quarter of the moves (<= 16)
-      const int mm = sw_m, nleft = k0 - K0, ncols = nleft + (Kend - c1);
-      const int q4 = tid & 3, c = tid >> 2;
-      const bool live = c < ncols;
-      const int col = c < nleft ? K0 + c : c1 + (c - nleft);
-      T v[16];
-#pragma unroll
-      for (int u = 0; u < 16; u++) {
-        const int q = q4 + 4 * u;
-        v[u] = (live && q < mm) ? A[(int64_t)sw_src[q] * n + col] : T(0);
+      const int lg = kw > 1 ? 32 - __clz(kw - 1) : 0;
+      for (int idx = tid; idx < (m << lg); idx += BT) {
+        const int d = idx >> lg, c = idx & ((1 << lg) - 1);
+        if (c < kw) A[(int64_t)(k0 + d) * n + k0 + c] = panel_value(lb, mp, urow, W, sh.src, d, c);
       }
-      __syncthreads();
-#pragma unroll
-      for (int u = 0; u < 16; u++) {
-        const int q = q4 + 4 * u;
-        if (live && q < mm) A[(int64_t)sw_dst[q] * n + col] = v[u];
-      }
-      __syncthreads();
     }
-    if (c1 < Kend) {
-      u_rows<T>(A, n, k0, kw, c1, Kend, panel, ld);
-      __syncthreads();
-      update_block<T, 256, 32>(A, n, c1, n, c1, Kend, k0, kw, smem);
-      continue;
-    }
-    // the outer block's last panel: its interchanges on the other columns
-    if (tid < 32) {
-      const int mm = compose_moves(piv, K0, Kend - K0, s_pos, s_cont, s_mdst, s_msrc);
-      if (tid == 0) sw_m = mm;
-    }
+    if (tid == 0) sh.mv_n = 0;
     __syncthreads();
-    apply_moves<T>(A, n, s_mdst, s_msrc, sw_m, 0, K0, reinterpret_cast<T*>(smem));
-    apply_moves<T>(A, n, s_mdst, s_msrc, sw_m, Kend, n, reinterpret_cast<T*>(smem));
-    if (Kend >= n) break;
-    T* dg = reinterpret_cast<T*>(smem);  // [32][33]: one diagonal block of L11
-    for (int q0 = K0; q0 < Kend; q0 += nb) {
-      const int qw = min(nb, Kend - q0);
-      for (int idx = tid; idx < qw * qw; idx += BT) {
-        const int i = idx / qw, p = idx - i * qw;
-        dg[i * 33 + p] = A[(int64_t)(q0 + i) * n + q0 + p];
-      }
-      __syncthreads();
-      u_rows<T>(A, n, q0, qw, Kend, n, dg, 33);
-      __syncthreads();
-      update_block<T, 32, 256>(A, n, q0 + qw, Kend, Kend, n, q0, qw, smem);
-    }
-    update_block<T, 64, 128>(A, n, Kend, n, Kend, n, K0, Kend - K0, smem);
+    list_moves(sh, sh.src, m, k0);
+    __syncthreads();
+    apply_moves<T, 16>(A, n, 1, sh, K0, k0, c1, Kend);
+    compose_map(sh, sh.ob, K0);
+    __syncthreads();
+    if (c1 < Kend) continue;
+    // ---- the outer block is done
+    if (tid == 0) sh.mv_n = 0;
+    __syncthreads();
+    list_moves(sh, sh.ob, n - K0, K0);
+    for (int d = tid; d < n - K0; d += BT)
+      if (sh.ob[d] < NB) sh.to[sh.ob[d]] = (unsigned short)(K0 + d);
+    __syncthreads();
+    apply_moves<T, 16>(A, n, 1, sh, 0, K0, K0, K0);
+    compose_map(sh, sh.perm, 0);
+    __syncthreads();
+    if (Kend < n) outer_update<T>(A, n, K0, nb, smem, sh);
   }
   return info;
 }
 
-// perm[i] = the original row that the interchanges j <-> piv[j] (j = 0 ..
-// n-1, in order) bring to row i; piv is copied to shared memory (scratch, n
-// ints) and one thread composes the sequence there.
-__device__ void pivots_to_perm(const int* piv, int n, int* perm, int* scratch) {
-  const int tid = threadIdx.x;
-  for (int i = tid; i < n; i += BT) {
-    perm[i] = i;
-    scratch[i] = piv[i];
+// Blocked forward (unit L) and backward (U) substitution, x in shared memory,
+// 32-row blocks: a warp-parallel product over the solved part (two rows of a
+// warp together), then one warp substitutes inside the 32 x 32 diagonal
+// block, staged in shared memory meanwhile.
+template <typename T>
+__device__ __forceinline__ void solve_block_dots(const T* LU, int n, const T* xs, int I0, int rows, int j0, int j1,
+                                                 BShared<T>& sh) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  T dg[2];
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    const int idx = tid + e * BT, i = idx >> 5, j = idx & 31;
+    dg[e] = (i < rows && j < rows) ? LU[(int64_t)(I0 + i) * n + I0 + j] : T(0);
+  }
+  const bool two = warp + NWARP < rows;
+  if (warp < rows) {
+    const T* ra = LU + (int64_t)(I0 + warp) * n;
+    const T* rb = LU + (int64_t)(I0 + (two ? warp + NWARP : warp)) * n;
+    T sa = 0, sb = 0;
+#pragma unroll 8
+    for (int j = j0 + lane; j < j1; j += 32) {
+      const T x = xs[j];
+      sa = fma(ra[j], x, sa);
+      sb = fma(rb[j], x, sb);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      sa += __shfl_xor_sync(0xffffffffu, sa, o);
+      sb += __shfl_xor_sync(0xffffffffu, sb, o);
+    }
+    if (lane == 0) {
+      sh.acc[warp] = sa;
+      if (two) sh.acc[warp + NWARP] = sb;
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    const int idx = tid + e * BT;
+    sh.diag[idx >> 5][idx & 31] = dg[e];
   }
   __syncthreads();
-  if (tid == 0)
-    for (int j = 0; j < n; j++) {
-      const int p = scratch[j];
-      if (p != j) {
-        const int t = perm[j];
-        perm[j] = perm[p];
-        perm[p] = t;
-      }
-    }
-  __syncthreads();
 }
 
-// x <- P x, x[i] <- x[perm[i]], through shared memory (buf: n elements)
 template <typename T>
-__device__ void gather_perm(T* x, int n, const int* perm, T* buf) {
-  for (int i = threadIdx.x; i < n; i += BT) buf[i] = x[perm[i]];
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += BT) x[i] = buf[i];
-  __syncthreads();
+__device__ void solve_system(const T* LU, int n, T* xs, BShared<T>& sh) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int I0 = 0; I0 < n; I0 += 32) {
+    const int rows = min(32, n - I0);
+    solve_block_dots(LU, n, xs, I0, rows, 0, I0, sh);
+    if (warp == 0) {
+      T v = lane < rows ? xs[I0 + lane] - sh.acc[lane] : T(0);
+      for (int j = 0; j < rows; j++) {
+        const T xj = __shfl_sync(0xffffffffu, v, j);
+        if (lane > j && lane < rows) v = fma(-sh.diag[lane][j], xj, v);
+      }
+      if (lane < rows) xs[I0 + lane] = v;
+    }
+    __syncthreads();
+  }
+  const int nblk = (n + 31) / 32;
+  for (int bi = nblk - 1; bi >= 0; bi--) {
+    const int I0 = bi * 32, rows = min(32, n - I0);
+    solve_block_dots(LU, n, xs, I0, rows, I0 + rows, n, sh);
+    if (warp == 0) {
+      T v = lane < rows ? xs[I0 + lane] - sh.acc[lane] : T(0);
+      for (int j = rows - 1; j >= 0; j--) {
+        if (lane == j) v = v / sh.diag[j][j];
+        const T xj = __shfl_sync(0xffffffffu, v, j);
+        if (lane < j) v = fma(-sh.diag[lane][j], xj, v);
+      }
+      if (lane < rows) xs[I0 + lane] = v;
+    }
+    __syncthreads();
+  }
 }
 
+// One CTA per SM; T: the type of the factors.  FP32: the copy of each matrix
+// is factored, then refined in FP64 against the matrix itself.
+template <typename T>
 __global__ void __launch_bounds__(BT, 1) batched_kernel(BatchArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ BShared<T> sh;
+  __shared__ int s_idx;
+  __shared__ double s_red[4][NWARP];
   WorkHeader* hdr = reinterpret_cast<WorkHeader*>(a.work);
   if (ld_acquire_s32(&hdr->bad) != 0) return;
   const int* order = reinterpret_cast<const int*>(a.work + hdr->order);
   const int64_t* offA32 = reinterpret_cast<const int64_t*>(a.work + hdr->offA32);
   const int64_t* offV = reinterpret_cast<const int64_t*>(a.work + hdr->offV);
-  int* pivs = reinterpret_cast<int*>(a.work + hdr->piv);
   float* A32s = reinterpret_cast<float*>(a.work + hdr->A32);
   double* r64s = reinterpret_cast<double*>(a.work + hdr->r64);
-  float* v32s = reinterpret_cast<float*>(a.work + hdr->v32);
-  __shared__ double sv_d[NWARP];
-  __shared__ float sv_f[NWARP];
-  __shared__ int sr[NWARP];
-  __shared__ int piv_s[kBatchMaxN];
-  __shared__ double s_acc_d[32];
-  __shared__ float s_acc_f[32];
-  __shared__ int s_idx;
-  __shared__ double s_red[4][NWARP];
   const int tid = threadIdx.x;
   for (;;) {
     if (tid == 0) s_idx = (int)atomicAdd(&hdr->queue, 1u);
@@ -646,57 +1022,85 @@ __global__ void __launch_bounds__(BT, 1) batched_kernel(BatchArgs a) {
     const int n = a.n[sys];
     double* A = a.A + a.a_off[sys];
     double* b = a.b + a.b_off[sys];
-    int* piv = pivs + offV[sys];
     int info = 0;
-    if (a.precision == LU_PREC_FP64) {
-      info = factor_system<double>(A, n, piv, smem, sv_d, sr, piv_s);
+    if constexpr (sizeof(T) == 8) {
+      info = factor_system<double>(A, n, smem, sh);
       __syncthreads();
-      pivots_to_perm(piv, n, piv_s, reinterpret_cast<int*>(smem));
-      gather_perm<double>(b, n, piv_s, reinterpret_cast<double*>(smem));
-      solve_global<double>(A, n, b, s_acc_d);
+      double* xs = reinterpret_cast<double*>(smem);
+      for (int i = tid; i < n; i += BT) xs[i] = b[sh.perm[i]];
+      __syncthreads();
+      solve_system<double>(A, n, xs, sh);
+      for (int i = tid; i < n; i += BT) b[i] = xs[i];
     } else {
       float* A32 = A32s + offA32[sys];
-      float* v = v32s + offV[sys];
       double* r = r64s + 2 * offV[sys];  // [r | b] per system
-      for (int idx = tid; idx < n * n; idx += BT) A32[idx] = (float)A[idx];
-      for (int i = tid; i < n; i += BT) {
-        r[n + i] = b[i];  // keep b for the residual
-        v[i] = (float)b[i];
+      for (int base = tid; base < n * n; base += 16 * BT) {  // 16 loads in flight per thread
+        double w[16];
+#pragma unroll
+        for (int e = 0; e < 16; e++) w[e] = base + e * BT < n * n ? A[base + e * BT] : 0.0;
+#pragma unroll
+        for (int e = 0; e < 16; e++)
+          if (base + e * BT < n * n) A32[base + e * BT] = (float)w[e];
       }
+      for (int i = tid; i < n; i += BT) r[n + i] = b[i];  // keep b for the residual
       __syncthreads();
-      info = factor_system<float>(A32, n, piv, smem, sv_f, sr, piv_s);
+      info = factor_system<float>(A32, n, smem, sh);
       __syncthreads();
-      // piv_s keeps the permutation for the refinement steps
-      pivots_to_perm(piv, n, piv_s, reinterpret_cast<int*>(smem));
-      gather_perm<float>(v, n, piv_s, reinterpret_cast<float*>(smem));
-      solve_global<float>(A32, n, v, s_acc_f);
+      double* x = reinterpret_cast<double*>(smem);        // [n] the solution
+      float* v = reinterpret_cast<float*>(x + kBatchMaxN);  // [n] the correction
+      for (int i = tid; i < n; i += BT) v[i] = (float)b[sh.perm[i]];
+      __syncthreads();
+      solve_system<float>(A32, n, v, sh);
       // x = v, then FP64 refinement: r = b - A x (against the FP64 A), stop
       // when the scaled residual r_hpl < 16, else v = P r, FP32 solve, x += v
-      for (int i = tid; i < n; i += BT) b[i] = (double)v[i];
+      for (int i = tid; i < n; i += BT) x[i] = (double)v[i];
       __syncthreads();
       const int warp = tid >> 5, lane = tid & 31;
       double anorm = 0.0, bmax = 0.0;
       for (int step = 0;; step++) {
         double rmax = 0.0, xmax = 0.0, an = 0.0;
-        for (int i = warp; i < n; i += NWARP) {
-          const double* row = A + (int64_t)i * n;
-          double acc = 0.0, as = 0.0;
-          for (int j = lane; j < n; j += 32) {
-            acc = fma(row[j], b[j], acc);
-            if (step == 0) as += fabs(row[j]);
+        for (int i = warp; i < n; i += 2 * NWARP) {  // two rows of a warp together
+          const bool two = i + NWARP < n;
+          const double* ra = A + (int64_t)i * n;
+          const double* rb = A + (int64_t)(two ? i + NWARP : i) * n;
+          double aa = 0.0, ab = 0.0, sa = 0.0, sb = 0.0;
+          if (step == 0) {
+#pragma unroll 4
+            for (int j = lane; j < n; j += 32) {
+              const double va = ra[j], vb = rb[j], xj = x[j];
+              aa = fma(va, xj, aa);
+              ab = fma(vb, xj, ab);
+              sa += fabs(va);
+              sb += fabs(vb);
+            }
+          } else {
+#pragma unroll 8
+            for (int j = lane; j < n; j += 32) {
+              const double xj = x[j];
+              aa = fma(ra[j], xj, aa);
+              ab = fma(rb[j], xj, ab);
+            }
           }
           for (int o = 16; o > 0; o >>= 1) {
-            acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            as += __shfl_xor_sync(0xffffffffu, as, o);
+            aa += __shfl_xor_sync(0xffffffffu, aa, o);
+            ab += __shfl_xor_sync(0xffffffffu, ab, o);
+            sa += __shfl_xor_sync(0xffffffffu, sa, o);
+            sb += __shfl_xor_sync(0xffffffffu, sb, o);
           }
           if (lane == 0) {
-            const double ri = r[i + n] - acc;  // r[n + i] keeps b
+            const double ri = r[i + n] - aa;  // r[n + i] keeps b
             r[i] = ri;
             rmax = fmax(rmax, fabs(ri));
-            an = fmax(an, as);
+            an = fmax(an, sa);
+            if (two) {
+              const double rj = r[i + NWARP + n] - ab;
+              r[i + NWARP] = rj;
+              rmax = fmax(rmax, fabs(rj));
+              an = fmax(an, sb);
+            }
           }
         }
-        for (int i = tid; i < n; i += BT) xmax = fmax(xmax, fabs(b[i]));
+        for (int i = tid; i < n; i += BT) xmax = fmax(xmax, fabs(x[i]));
         if (step == 0)
           for (int i = tid; i < n; i += BT) bmax = fmax(bmax, fabs(r[i + n]));
         // block maxima
@@ -736,12 +1140,13 @@ __global__ void __launch_bounds__(BT, 1) batched_kernel(BatchArgs a) {
           if (tid == 0) atomicAdd(&hdr->refine_hist[kRefineHistBins - 1], 1);
           break;
         }
-        for (int i = tid; i < n; i += BT) v[i] = (float)r[piv_s[i]];
+        for (int i = tid; i < n; i += BT) v[i] = (float)r[sh.perm[i]];
         __syncthreads();
-        solve_global<float>(A32, n, v, s_acc_f);
-        for (int i = tid; i < n; i += BT) b[i] += (double)v[i];
+        solve_system<float>(A32, n, v, sh);
+        for (int i = tid; i < n; i += BT) x[i] += (double)v[i];
         __syncthreads();
       }
+      for (int i = tid; i < n; i += BT) b[i] = x[i];
     }
     if (tid == 0) a.info[sys] = info;
     __syncthreads();
@@ -887,8 +1292,10 @@ extern "C" LU_API int lu_batched_factor_solve(int32_t count, const int32_t* n, c
   cudaStream_t s = (cudaStream_t)stream;
   static PerDeviceOnce once;
   LUB_TRY(once_per_device(once, [] {
+    LUB_TRY(cuda_status(cudaFuncSetAttribute(batched_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kBatchSmem)));
     return cuda_status(
-        cudaFuncSetAttribute(batched_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchSmem));
+        cudaFuncSetAttribute(batched_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBatchSmem));
   }));
   unsigned char* w = static_cast<unsigned char*>(dWork);
   batched_prep_kernel<<<1, 1024, 0, s>>>(count, n, precision, w, (long long)work_bytes, info);
@@ -897,7 +1304,10 @@ extern "C" LU_API int lu_batched_factor_solve(int32_t count, const int32_t* n, c
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   BatchArgs a{count, n, a_off, b_off, dA, db, info, precision, w};
-  batched_kernel<<<std::min(count, sms), BT, kBatchSmem, s>>>(a);
+  if (precision == LU_PREC_FP64)
+    batched_kernel<double><<<std::min(count, sms), BT, kBatchSmem, s>>>(a);
+  else
+    batched_kernel<float><<<std::min(count, sms), BT, kBatchSmem, s>>>(a);
   LUB_LAUNCH_CHECK();
   return LU_OK;
 }

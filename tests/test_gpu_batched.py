@@ -131,3 +131,67 @@ def test_batched_rejects_bad_order(cuda_dev):
     torch.cuda.synchronize()
     assert rc == 0
     assert np.all(info.cpu().numpy() == -1)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_batched_edges_of_blocks_and_tiles(cuda_dev, prec):
+    """Orders at the edges of the kernel's shapes: panel widths, the shared-memory
+    threshold, outer blocks of 64 / 128, 64- and 128-wide tiles, 512 and 1024
+    panel rows.  FP64 factors against the bound |P A - L U| <= gamma_n |L||U|
+    (elimination, each update one fma or a sum of products subtracted once: at
+    most n roundings per element, Higham theorem 9.3), solutions by r_hpl < 16."""
+    import scipy.linalg
+    from charmlu_b200 import LU_PREC_FP32, LU_PREC_FP64
+    from charmlu_b200.batched import BatchedSystems
+    ns = [1, 2, 3, 15, 16, 17, 31, 33, 63, 64, 65, 95, 97, 127, 128, 129, 159, 160, 161, 191, 193, 255, 257, 320, 383,
+          385, 511, 512, 513, 577, 650, 652, 769, 1023, 1025]
+    rng = np.random.default_rng(11)
+    mats = [rng.uniform(-0.5, 0.5, (n, n)) for n in ns]
+    rhs = [rng.uniform(-0.5, 0.5, n) for n in ns]
+    bs = BatchedSystems(ns)
+    A = torch.from_numpy(np.concatenate([m.ravel() for m in mats])).cuda()
+    b = torch.from_numpy(np.concatenate(rhs)).cuda()
+    info = bs.factor_solve(A, b, LU_PREC_FP64 if prec == "fp64" else LU_PREC_FP32).cpu().numpy()
+    assert (info == 0).all()
+    x, F = b.cpu().numpy(), A.cpu().numpy()
+    u = 2.0 ** -53
+    for i, n in enumerate(ns):
+        xi = x[bs.b_off[i]:bs.b_off[i] + n]
+        r = np.abs(rhs[i] - mats[i] @ xi).max()
+        assert r < 16 * n * 2 * u * (np.abs(mats[i]).sum(1).max() * np.abs(xi).max() + np.abs(rhs[i]).max()), n
+        if prec == "fp64":
+            LU = F[bs.a_off[i]:bs.a_off[i] + n * n].reshape(n, n)
+            L = np.tril(LU, -1) + np.eye(n)
+            U = np.triu(LU)
+            assert np.abs(L).max() <= 1, n
+            _, piv = scipy.linalg.lu_factor(mats[i])
+            P = np.arange(n)
+            for j, p in enumerate(piv):
+                P[[j, p]] = P[[p, j]]
+            # the products below round too (in FP64): n more roundings
+            bound = 2 * (n + 1) * u / (1 - 2 * (n + 1) * u) * (np.abs(L) @ np.abs(U)) + u
+            assert (np.abs(mats[i][P] - L @ U) <= bound).all(), n
+        else:
+            np.testing.assert_array_equal(F[bs.a_off[i]:bs.a_off[i] + n * n], mats[i].ravel())
+
+
+def test_batched_singular_and_ties(cuda_dev):
+    """A zero column is reported at its place; all-equal candidates take the lowest row."""
+    from charmlu_b200 import LU_PREC_FP64
+    from charmlu_b200.batched import BatchedSystems
+    ns = [20, 70, 200, 300]
+    rng = np.random.default_rng(3)
+    mats = []
+    for n in ns:
+        m = rng.uniform(-0.5, 0.5, (n, n))
+        m[:, n // 2] = 0
+        mats.append(m)
+    eye = [np.eye(n) for n in ns]  # every step has one candidate; no interchange, x = b
+    bs = BatchedSystems(ns + ns)
+    A = torch.from_numpy(np.concatenate([m.ravel() for m in mats + eye])).cuda()
+    rhs = np.concatenate([rng.uniform(-0.5, 0.5, n) for n in ns + ns])
+    b = torch.from_numpy(rhs).cuda()
+    info = bs.factor_solve(A, b, LU_PREC_FP64).cpu().numpy()
+    assert info.tolist() == [n // 2 + 1 for n in ns] + [0] * 4
+    o = int(bs.b_off[4])
+    np.testing.assert_array_equal(b.cpu().numpy()[o:], rhs[o:])
