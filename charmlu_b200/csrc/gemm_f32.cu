@@ -110,10 +110,11 @@ gemm_f32_sub_kernel(const float* __restrict__ A, int64_t lda, const float* __res
 // These launches are bound by the M x K and M x N traffic, which the 128 x
 // 128 tile above would spend mostly on zero-filled columns.  Each element is
 // accumulated over k in the same order and subtracted once, as above, so
-// both kernels give the same bits.
+// both kernels give the same bits.  CHAIN: C is the start of each sum instead
+// and A enters negated, one fma per k, as elimination column by column does.
 constexpr int NBM = 64, NKMAX = 64, NTHREADS = 256;
 
-template <int BN>
+template <int BN, bool CHAIN = false>
 __global__ void __launch_bounds__(NTHREADS)
 gemm_f32_narrow_kernel(const float* __restrict__ A, int64_t lda, const float* __restrict__ B, int64_t ldb,
                        float* __restrict__ C, int64_t ldc, int M, int N, int K) {
@@ -138,12 +139,15 @@ gemm_f32_narrow_kernel(const float* __restrict__ A, int64_t lda, const float* __
 #pragma unroll
   for (int i = 0; i < RPT; i++)
 #pragma unroll
-    for (int e = 0; e < 4; e++) acc[i][e] = 0.f;
+    for (int e = 0; e < 4; e++) {
+      const int r = row0 + ty + i * RG, c = tx * 4 + e;
+      acc[i][e] = CHAIN && r < M && c < N ? C[(int64_t)r * ldc + c] : 0.f;
+    }
   for (int k = 0; k < K; k++) {
     const float4 b = *reinterpret_cast<const float4*>(&Bs[k][tx * 4]);
 #pragma unroll
     for (int i = 0; i < RPT; i++) {
-      const float a = As[ty + i * RG][k];
+      const float a = CHAIN ? -As[ty + i * RG][k] : As[ty + i * RG][k];
       acc[i][0] = fmaf(a, b.x, acc[i][0]);
       acc[i][1] = fmaf(a, b.y, acc[i][1]);
       acc[i][2] = fmaf(a, b.z, acc[i][2]);
@@ -157,7 +161,10 @@ gemm_f32_narrow_kernel(const float* __restrict__ A, int64_t lda, const float* __
 #pragma unroll
     for (int e = 0; e < 4; e++) {
       const int c = tx * 4 + e;
-      if (c < N) C[(int64_t)r * ldc + c] -= acc[i][e];
+      if (c < N) {
+        if (CHAIN) C[(int64_t)r * ldc + c] = acc[i][e];
+        else C[(int64_t)r * ldc + c] -= acc[i][e];
+      }
     }
   }
 }
@@ -184,6 +191,15 @@ static int gemm_f32_dispatch(const float* A, int64_t lda, const float* B, int64_
 int launch_gemm_f32_sub(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc, int M,
                         int N, int K, cudaStream_t s) {
   return gemm_f32_dispatch(A, lda, B, ldb, C, ldc, M, N, K, true, s);
+}
+
+int launch_gemm_f32_chain(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc, int M,
+                          int N, int K, cudaStream_t s) {
+  if (M <= 0 || N <= 0 || K <= 0) return LU_OK;
+  if (N > 32 || K > NKMAX) return LU_ERR_ARG;
+  gemm_f32_narrow_kernel<32, true><<<ceil_div(M, NBM), NTHREADS, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K);
+  LUB_LAUNCH_CHECK();
+  return LU_OK;
 }
 
 }  // namespace lub

@@ -55,8 +55,13 @@ struct lu_handle_s {
   // columns first, the rest after the panel has started (LU_B200_LA_SPLIT)
   int la_split = 1;  // mixed look-ahead: the next panel's columns first, then the rest
   // leaf tuning: recursion leaf width and CTA cap, without / with look-ahead
-  int leaf_w64 = 32, leaf_w32 = 32, leaf_ctas = 148;
+  int leaf_w64 = 32, leaf_w32 = 64, leaf_ctas = 148;
   int leaf_w64_la = 16, leaf_w32_la = 32, leaf_ctas_la = 48;
+  // look-ahead is used while more than this many rows are left
+  // (LU_B200_LA_MIN).  B200: FP64 n = 4999 23.1 ms with look-ahead to the end,
+  // 19.5 without; n = 16384 141.8 / 137.4 with 6144 / 141.9 with 10240; mixed
+  // n = 8192 30.2 / 22.4; n = 32768 179 / 171 with 16384 / 182 with 24576
+  int la_min64 = 6144, la_min32 = 16384;
   // low-precision trailing update: CTAs of the persistent kernel (0: one CTA
   // per tile); under look-ahead the update beside a running panel leaves
   // gemm_reserve SMs to it

@@ -22,6 +22,11 @@ int launch_gemm_f64_sub(const CUtensorMap& mapA, const CUtensorMap& mapB, const 
 int launch_gemm_f32_sub(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc, int M,
                         int N, int K, cudaStream_t s);
 
+// The same for N <= 32, K <= 64 with one fma per k starting from C, the order of
+// column-by-column elimination
+int launch_gemm_f32_chain(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc, int M,
+                          int N, int K, cudaStream_t s);
+
 // ---- unblocked panel leaf (rows resident in registers)
 constexpr int kMaxLeafCTAs = 160;
 constexpr int kMaxLeafW = 64;         // tournament leaf's scratch

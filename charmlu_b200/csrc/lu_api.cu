@@ -95,6 +95,7 @@ struct Ctx64 {
   PivotList pl;
   int leaf_w;
   int leaf_ctas;
+  bool alone = true;  // no kernel of another stream runs beside the panel
   int base = 0;  // global row/column of the matrix's first row (a panel view)
 };
 
@@ -143,7 +144,7 @@ int panel64(Ctx64& c, int c0, int w, int p0, int pw) {
     if (!tag) return LU_ERR_NOMEM;
     Prof pf(c.h, c.s, LU_PH_PANEL, (double)M * w * w);
     return launch_getf2_leaf<double>(c.A.at(c0, c0), c.A.ld, M, w, c.ipiv + c0, c.base + c0, c.h->leaf_pkt, tag,
-                                     c.h->st, c.base + c0, c.thr, c.h->spin, c.leaf_ctas, !c.h->cfg.lookahead, c.s,
+                                     c.h->st, c.base + c0, c.thr, c.h->spin, c.leaf_ctas, c.alone, c.s,
                                      c.A.at(c0, p0), pw, c0 - p0);
   }
   const int w1 = split_w(w), w2 = w - w1;
@@ -174,17 +175,18 @@ int factor_f64_schedule(lu_handle h, double* dA, int64_t lda, int32_t* ipiv, dou
   const bool la = h->cfg.lookahead != 0;
   Ctx64 c;
   c.h = h; c.ipiv = ipiv; c.n = n; c.s = s; c.thr = h->cfg.sing_threshold; c.pl = h->plist;
-  c.leaf_w = la ? h->leaf_w64_la : h->leaf_w64;
-  c.leaf_ctas = la ? h->leaf_ctas_la : h->leaf_ctas;
+  c.leaf_w = la ? h->leaf_w64_la : h->leaf_w64;  // one width per factorisation: the same bits wherever the schedule changes
+  c.leaf_ctas = h->leaf_ctas;
   LUB_TRY(c.A.init(dA, n, n, lda));
   LUB_CUDA(cudaMemsetAsync(h->st, 0, sizeof(DevStatus), s));
   LUB_CUDA(cudaMemsetAsync(h->leaf_pkt, 0, h->clear_bytes(), s));
   h->next_counter = 0;
   LUB_TRY(launch_iota(h->perm, n, s));
-  if (!la) {
-    for (int k0 = 0; k0 < n; k0 += b) {
+  // panel at k0 (unless it is factored already), then its step, and so on
+  auto in_sequence = [&](int k0, bool factored) {
+    for (; k0 < n; k0 += b, factored = false) {
       const int kw = std::min(b, n - k0);
-      LUB_TRY(panel64(c, k0, kw, k0, kw));
+      if (!factored) LUB_TRY(panel64(c, k0, kw, k0, kw));
       LUB_TRY(pivots_apply_f64(c, k0, kw, 0, n, k0, k0 + kw, rhs, h->perm));
       const int rest = n - k0 - kw;
       if (rest > 0) {
@@ -192,15 +194,21 @@ int factor_f64_schedule(lu_handle h, double* dA, int64_t lda, int32_t* ipiv, dou
         LUB_TRY(gemm64(c, c.A, k0 + kw, k0 + kw, c.A, k0 + kw, k0, c.A, k0, k0 + kw, rest, rest, kw, LU_PH_GEMM));
       }
     }
-    return LU_OK;
-  }
+    return (int)LU_OK;
+  };
+  if (!la || n <= h->la_min64) return in_sequence(0, false);
   // Look-ahead (replaces BlockScheduler's policy, scheduler.C:235-484, and the
   // eager U solve next to the diagonal, lu.ci:141-145): panel k+1 runs on the
   // high-priority panel stream as soon as the trailing update has reached its
   // columns, while the rest of trailing update k runs on the caller's stream.
+  // Once la_min64 rows or fewer are left, the update is too short to hide a
+  // panel and the panel is faster with the GPU to itself (one cluster): the
+  // rest runs in sequence.
   Ctx64 cp = c;
   cp.s = h->sP;
   cp.pl = h->plistP;
+  cp.leaf_ctas = h->leaf_ctas_la;
+  cp.alone = false;
   // under capture the panel stream's kernel nodes are marked for its priority
   std::vector<cudaGraphNode_t> mark;
   LUB_CUDA(cudaEventRecord(h->evFork, s));
@@ -212,6 +220,7 @@ int factor_f64_schedule(lu_handle h, double* dA, int64_t lda, int32_t* ipiv, dou
   for (int k0 = 0; k0 < n; k0 += b) {
     const int kw = std::min(b, n - k0), k1 = k0 + kw, rest = n - k1;
     LUB_CUDA(cudaStreamWaitEvent(s, h->evP, 0));  // panel k factored (joins the panel stream)
+    if (rest <= h->la_min64) return in_sequence(k0, true);
     LUB_TRY(pivots_apply_f64(c, k0, kw, 0, n, k0, k1, rhs, h->perm));
     if (rest <= 0) continue;
     LUB_TRY(trsm64(c, c.A, k0, kw, c.A, k0, k1, rest));
@@ -323,14 +332,15 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
   if (const char* e = getenv("LU_B200_LEAF_CTAS_LA")) h->leaf_ctas_la = std::max(1, atoi(e));
   if (const char* e = getenv("LU_B200_LEAF_W64")) h->leaf_w64 = std::min(32, std::max(2, atoi(e)));
   if (const char* e = getenv("LU_B200_LEAF_W64_LA")) h->leaf_w64_la = std::min(32, std::max(2, atoi(e)));
-  if (const char* e = getenv("LU_B200_LEAF_W32")) h->leaf_w32 = std::min(32, std::max(4, atoi(e)));
-  if (const char* e = getenv("LU_B200_LEAF_W32_LA")) h->leaf_w32_la = std::min(32, std::max(4, atoi(e)));
+  if (const char* e = getenv("LU_B200_LEAF_W32")) h->leaf_w32 = std::min(64, std::max(4, atoi(e)));
+  if (const char* e = getenv("LU_B200_LEAF_W32_LA")) h->leaf_w32_la = std::min(64, std::max(4, atoi(e)));
   if (const char* e = getenv("LU_B200_GEMM_CTAS")) h->gemm_ctas = std::max(0, atoi(e));
   if (const char* e = getenv("LU_B200_GEMM_RESERVE")) h->gemm_reserve = std::max(0, atoi(e));
   if (const char* e = getenv("LU_B200_GEMM_HELPER")) h->gemm_helper = atoi(e) != 0;
   if (const char* e = getenv("LU_B200_GEMM_PAIR")) h->gemm_pair = atoi(e) != 0;
   if (const char* e = getenv("LU_B200_PANEL_TC")) h->panel_tc = atoi(e) != 0;
   if (const char* e = getenv("LU_B200_LA_SPLIT")) h->la_split = atoi(e) != 0;
+  if (const char* e = getenv("LU_B200_LA_MIN")) h->la_min64 = h->la_min32 = std::max(0, atoi(e));
   if (const char* e = getenv("LU_B200_TSLU")) h->tslu = atoi(e) != 0;
   if (const char* e = getenv("LU_B200_TRSM_BLOCK")) h->trsm_block = std::max(0, std::min(2, atoi(e)));
   if (const char* e = getenv("LU_B200_TRSM_WIDE")) h->trsm_wide = atoi(e) != 0;
@@ -628,6 +638,7 @@ Ctx64 block_ctx(lu_handle h, cudaStream_t s) {
   c.pl = h->plist;
   c.leaf_w = la ? h->leaf_w64_la : h->leaf_w64;
   c.leaf_ctas = la ? h->leaf_ctas_la : h->leaf_ctas;
+  c.alone = !la;
   return c;
 }
 

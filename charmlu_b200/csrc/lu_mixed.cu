@@ -98,6 +98,7 @@ struct Ctx32 {
   PivotList pl;
   int leaf_w;
   int leaf_ctas;
+  bool alone = true;  // no kernel of another stream runs beside the panel
 };
 
 inline int split_w32(int w) {
@@ -180,18 +181,33 @@ int panel_gemm_tc(Ctx32& c, int r0, int M, int kc, int K, int n0, int N, int cen
 // the leaves swap rows across the whole panel (no laswp in the recursion)
 int panel32(Ctx32& c, int c0, int w, int p0, int pw) {
   const int M = c.n - c0;
-  if (w <= std::min(c.leaf_w, leaf_max_width<float>(M, c.h->num_sms))) {
-    Prof pf(c.h, c.s, LU_PH_PANEL, (double)M * w * w);
-    if (c.h->tslu && c.h->tslu_scr.cand_idx) {
-      const int rc = launch_tslu_leaf(c.A + (int64_t)c0 * c.ld + c0, c.ld, M, w, c.ipiv + c0, c0, c.h->tslu_scr,
-                                      c.h->st, c0, c.thr, c.leaf_ctas, c.s, c.A + (int64_t)c0 * c.ld + p0, pw, c0 - p0);
-      if (rc != LU_ERR_UNSUPPORTED) return rc;
-    }
+  auto at = [&](int r, int cc) { return c.A + (int64_t)r * c.ld + cc; };
+  auto leaf = [&](int l0, int lw) {
     const unsigned tag = c.h->take_leaf_tag();
-    if (!tag) return LU_ERR_NOMEM;
-    return launch_getf2_leaf<float>(c.A + (int64_t)c0 * c.ld + c0, c.ld, M, w, c.ipiv + c0, c0, c.h->leaf_pkt, tag,
-                                    c.h->st, c0, c.thr, c.h->spin, c.leaf_ctas, !c.h->cfg.lookahead, c.s,
-                                    c.A + (int64_t)c0 * c.ld + p0, pw, c0 - p0);
+    if (!tag) return (int)LU_ERR_NOMEM;
+    return launch_getf2_leaf<float>(at(l0, l0), c.ld, c.n - l0, lw, c.ipiv + l0, l0, c.h->leaf_pkt, tag, c.h->st, l0,
+                                    c.thr, c.h->spin, c.leaf_ctas, c.alone, c.s, at(l0, p0), pw, l0 - p0);
+  };
+  const int lmax = leaf_max_width<float>(M, c.h->num_sms);
+  if (c.h->tslu && c.h->tslu_scr.cand_idx && w <= std::min(c.leaf_w, 32)) {
+    Prof pf(c.h, c.s, LU_PH_PANEL, (double)M * w * w);
+    const int rc = launch_tslu_leaf(at(c0, c0), c.ld, M, w, c.ipiv + c0, c0, c.h->tslu_scr, c.h->st, c0, c.thr,
+                                    c.leaf_ctas, c.s, at(c0, p0), pw, c0 - p0);
+    if (rc != LU_ERR_UNSUPPORTED) return rc;
+  }
+  if (w <= std::min(c.leaf_w, lmax)) {
+    Prof pf(c.h, c.s, LU_PH_PANEL, (double)M * w * w);
+    return leaf(c0, w);
+  }
+  if (w <= c.leaf_w && w <= 64 && lmax == 32 && !c.h->tslu) {
+    // a leaf of up to 64 columns as two of at most 32, the second brought up to
+    // date by one fma per column, in column order: the bits of one leaf
+    Prof pf(c.h, c.s, LU_PH_PANEL, (double)M * w * w);
+    const int c1 = c0 + 32, w2 = w - 32;
+    LUB_TRY(leaf(c0, 32));
+    LUB_TRY(launch_trsm_llu_leaf<float>(at(c0, c0), c.ld, at(c0, c1), c.ld, 32, w2, c.s));
+    LUB_TRY(launch_gemm_f32_chain(at(c1, c0), c.ld, at(c0, c1), c.ld, at(c1, c1), c.ld, M - 32, w2, 32, c.s));
+    return leaf(c1, w2);
   }
   const int w1 = split_w32(w), w2 = w - w1;
   LUB_TRY(panel32(c, c0, w1, p0, pw));
@@ -353,34 +369,52 @@ int factor_mixed(lu_handle h, cudaStream_t s, const double* rest_src, int64_t re
   const int n = (int)h->cfg.n, B = h->cfg.block_size;
   const bool bf16 = h->cfg.precision == LU_PREC_BF16;
   const bool la = h->cfg.lookahead != 0;
-  // the tournament-pivoting leaf handles widths up to 32
-  const int lw = la ? h->leaf_w32_la : h->leaf_w32;
   Ctx32 c{h, h->A32, h->ld32, n, h->ipiv32, s, h->cfg.sing_threshold, h->plist,
-          h->tslu ? std::min(lw, 32) : lw, la ? h->leaf_ctas_la : h->leaf_ctas};
+          la ? h->leaf_w32_la : h->leaf_w32, h->leaf_ctas};
   CUtensorMap mapC;
   LUB_TRY(encode_tmap_2d(&mapC, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, h->A32, n, n, h->ld32 * 4, 32, 128,
                          CU_TENSOR_MAP_SWIZZLE_128B));
   LUB_CUDA(cudaMemsetAsync(h->leaf_pkt, 0, h->clear_bytes(), s));
   h->next_counter = 0;
   LUB_TRY(launch_iota(h->perm, n, s));
-  if (!la) {
-    for (int k0 = 0; k0 < n; k0 += B) {
+  const bool split = la && h->la_split && h->pairs && !bf16;
+  // panel at k0 (unless it is factored already), then its step, and so on
+  auto in_sequence = [&](int k0, bool factored) {
+    for (; k0 < n; k0 += B, factored = false) {
       const int kw = std::min(B, n - k0);
-      LUB_TRY(panel32(c, k0, kw, k0, kw));
+      if (!factored) LUB_TRY(panel32(c, k0, kw, k0, kw));
       LUB_TRY(pivots_apply_f32(c, k0, kw, 0, n, k0, k0 + kw, h->perm));
       const int k1 = k0 + kw, rest = n - k1;
       if (rest <= 0) continue;
-      LUB_TRY(trsm32(c, k0, kw, k0, k1, rest));
       CUtensorMap mapL, mapU;
       int K = 0, kpart = 0;
+      if (split) {  // in the parts of a split look-ahead step, each with its own scale: the same bits
+        const int nw = std::min(B, rest);
+        for (int part = 0; part < 2; part++) {
+          const int u0 = part ? nw : 0, nc = part ? rest - nw : nw;
+          unsigned* am = h->amax + 2 * part;
+          if (nc <= 0) break;
+          LUB_TRY(trsm32(c, k0, kw, k0, k1 + u0, nc));
+          LUB_TRY(build_operands_part(h, c, k0, kw, k1, rest, u0, nc, part == 0, am, &mapL, &mapU, &K, &kpart, s));
+          LUB_TRY(lowp_gemm(h, mapL, mapU, mapC, k1, rest, u0, nc, K, kpart, kw, false, s, 0, nullptr, 0, am));
+        }
+        continue;
+      }
+      LUB_TRY(trsm32(c, k0, kw, k0, k1, rest));
       LUB_TRY(build_operands(h, c, k0, kw, k1, rest, bf16, &mapL, &mapU, &K, &kpart, s));
       LUB_TRY(lowp_gemm(h, mapL, mapU, mapC, k1, rest, 0, rest, K, kpart, kw, bf16, s));
     }
-    return LU_OK;
-  }
+    return (int)LU_OK;
+  };
+  if (!la) return in_sequence(0, false);
+  // Once la_min32 rows or fewer are left, the update is too short to hide a
+  // panel and the panel is faster with the GPU to itself (one cluster up to
+  // 24576 rows): the rest runs in sequence.
   Ctx32 cp = c;
   cp.s = h->sP;
   cp.pl = h->plistP;
+  cp.leaf_ctas = h->leaf_ctas_la;
+  cp.alone = false;
   // under capture the panel stream's kernel nodes are marked for its priority
   std::vector<cudaGraphNode_t> mark;
   LUB_CUDA(cudaEventRecord(h->evFork, s));
@@ -393,10 +427,10 @@ int factor_mixed(lu_handle h, cudaStream_t s, const double* rest_src, int64_t re
     Prof pf(h, s, LU_PH_OTHER);
     LUB_TRY(launch_f64_to_f32(rest_src + B, rest_lda, h->A32 + B, h->ld32, n, n - B, s));
   }
-  const bool split = h->la_split && h->pairs && !bf16;
   for (int k0 = 0; k0 < n; k0 += B) {
     const int kw = std::min(B, n - k0), k1 = k0 + kw, rest = n - k1;
     LUB_CUDA(cudaStreamWaitEvent(s, h->evP, 0));
+    if (rest <= h->la_min32) return in_sequence(k0, true);
     if (split && rest > 0) {
       LUB_TRY(factor_mixed_split_step(h, c, cp, mapC, k0, kw, s));
       continue;
