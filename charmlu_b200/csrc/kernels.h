@@ -18,6 +18,14 @@ int gemm_f64_init();
 int gemm_f64_smem_bytes();
 int launch_gemm_f64_sub(const CUtensorMap& mapA, const CUtensorMap& mapB, const GemmArgs& a, cudaStream_t s);
 
+// C (M x N) -= A (M x K) B (K x N) in small tiles (few columns or few rows);
+// even leading dimensions, 16-byte aligned pointers
+int launch_gemm_f64_small(const double* A, int64_t lda, const double* B, int64_t ldb, double* C, int64_t ldc, int M,
+                          int N, int K, cudaStream_t s);
+// B (w x ncols) <- L^{-1} B, L unit lower, w <= 256, one launch; even leading
+// dimensions, 16-byte aligned pointers
+int launch_trsm_f64_strip(const double* L, int64_t ldl, double* B, int64_t ldb, int w, int ncols, cudaStream_t s);
+
 // FP32 SIMT GEMM C -= A * B (panel / TRSM halves of the mixed path)
 int launch_gemm_f32_sub(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc, int M,
                         int N, int K, cudaStream_t s);

@@ -114,6 +114,15 @@ int pivots_apply_f64(Ctx64& c, int k0, int cnt, int c_begin, int c_end, int skip
 int gemm64(Ctx64& c, const MatF64& Cm, int rc, int cc, const MatF64& Am, int ra, int ca, const MatF64& Bm, int rb,
            int cb, int M, int N, int K, int phase = LU_PH_GEMM_IN) {
   Prof pf(c.h, c.s, phase, 2.0 * M * (double)N * K);
+  // 64 x 32 tiles where half or more of a 128-wide tile's columns would be
+  // padding (n = 2048, b = 128: 5.01 -> 4.68 ms; n = 16384 135.4 -> 132.0) or
+  // where 128 x 128 tiles make fewer than two waves (2048: 4.68 -> 4.54; 16384:
+  // 132.0 -> 131.1); the same bits
+  const int64_t tiles = (int64_t)ceil_div(M, 128) * ceil_div(N, 128);
+  if (N <= 64 || tiles <= 2 * kNumSMsB200) {
+    if ((ca & 1) || (cb & 1) || (cc & 1)) return LU_ERR_ALIGN;
+    return launch_gemm_f64_small(Am.at(ra, ca), Am.ld, Bm.at(rb, cb), Bm.ld, Cm.at(rc, cc), Cm.ld, M, N, K, c.s);
+  }
   GemmArgs g;
   g.a_row0 = ra; g.a_col0 = ca; g.b_row0 = rb; g.b_col0 = cb;
   g.C = Cm.at(rc, cc); g.ldc = Cm.ld;
@@ -127,6 +136,10 @@ int trsm64(Ctx64& c, const MatF64& Lm, int r0, int w, const MatF64& Bm, int rb, 
   if (w <= 32) {
     Prof pf(c.h, c.s, LU_PH_TRSM, (double)w * w * ncols);
     return launch_trsm_llu_leaf<double>(Lm.at(r0, r0), Lm.ld, Bm.at(rb, cb), Bm.ld, w, ncols, c.s);
+  }
+  if (w <= 256 && !(r0 & 1) && !(cb & 1)) {
+    Prof pf(c.h, c.s, LU_PH_TRSM, (double)w * w * ncols);
+    return launch_trsm_f64_strip(Lm.at(r0, r0), Lm.ld, Bm.at(rb, cb), Bm.ld, w, ncols, c.s);
   }
   const int w1 = split_w(w);
   LUB_TRY(trsm64(c, Lm, r0, w1, Bm, rb, cb, ncols));
