@@ -26,8 +26,13 @@
 //     position it stands at, the chosen row leaves the set, the row standing
 //     at the diagonal takes the chosen row's position;
 //   * a CTA's candidate takes one barrier: each warp reduces its rows with
-//     redux on the bit patterns of |a| and its winner writes the whole row to
-//     shared memory, then a warp reduces the eight winners;
+//     redux on the bit patterns of |a|, then a warp reduces the eight winners.
+//     The best row reaches shared memory from the one lane that holds it, after
+//     the winner is known: one lane stores 4 bytes a cycle, and eight warps
+//     writing their candidates' rows ahead of the barrier took 290 - 520 cycles
+//     of a column (FP64 256 x 32 36.3 -> 30.8 us, cluster 2048 x 32 48.6 ->
+//     42.8).  In a grid, where L2 latency dominates and the row has to leave at
+//     once, they are written ahead (FP32 36864 x 32: 84.5 us, 90 the other way);
 //   * between CTAs there is no barrier.  In a cluster every CTA sends its
 //     candidate (header and row) to every peer with st.async and waits on its
 //     own mbarrier for G of them.  In a larger grid warp 0 publishes header
@@ -117,8 +122,11 @@ struct LeafArgs {
 
 template <typename T, int W, int RPT, int XP>
 struct LeafShared {
-  alignas(16) T row[2][NW][W];  // each warp's candidate row (rotated), by column parity
-  alignas(16) T urow[W][W];     // the chosen rows: element i of row j is column j + i
+  // row j: the row chosen in column j, element i of it being column j + i
+  // (cluster: this CTA's candidate, which is that row where it matters)
+  alignas(16) T urow[W][W];
+  // grid: each warp's candidate row, by column parity
+  alignas(16) T row[XP == kGrid ? 2 : 1][XP == kGrid ? NW : 1][W];
   alignas(16) T zero[W];
   // cluster: every CTA's candidate, by column parity
   alignas(16) T crow[XP == kCluster ? 2 : 1][XP == kCluster ? kMaxCluster : 1][W];
@@ -126,6 +134,7 @@ struct LeafShared {
   alignas(8) uint64_t bar[2];
   T key[2][NW];
   int pos[2][NW];
+  T piv[W];  // the chosen pivots
   int p[W];  // position chosen in column j; -1: none usable, -2: a wait ran out
   int src[W];
   int mv_dst[2 * W], mv_src[2 * W];
@@ -218,166 +227,173 @@ __global__ void __launch_bounds__(NT, 1) getf2_leaf_kernel(T* P, T* prow0, LeafA
   for (int j = 0; j < ncols; j++) {
     const int buf = j & 1;
     // ---- the CTA's candidate
-    {
-      T bv = 0;
-      int bp = -1, bu = 0;
+    T bv = 0;
+    int bp = -1, bu = 0;
 #pragma unroll
-      for (int u = 0; u < RPT; u++) {
-        const T x = fabs(v[u][0]);
-        if (pos[u] >= 0 && (x > bv || (x == bv && bp >= 0 && pos[u] < bp))) {
-          bv = x;
-          bp = pos[u];
-          bu = u;
-        }
-      }
-      const int wl = warp_best(bv, bp >= 0, bp);
-      if (lane == max(wl, 0)) {
-        sh.key[buf][warp] = bv;
-        sh.pos[buf][warp] = wl < 0 ? -1 : bp;
-#pragma unroll
-        for (int u = 0; u < RPT; u++)
-          if (RPT == 1 || bu == u) {
-#pragma unroll
-            for (int i = 0; i < W; i += V) {
-              int4 q;
-              memcpy(&q, &v[u][i], 16);
-              *reinterpret_cast<int4*>(&sh.row[buf][warp][i]) = q;
-            }
-          }
+    for (int u = 0; u < RPT; u++) {
+      const T x = fabs(v[u][0]);
+      if (pos[u] >= 0 && (x > bv || (x == bv && bp >= 0 && pos[u] < bp))) {
+        bv = x;
+        bp = pos[u];
+        bu = u;
       }
     }
+    const int wl = warp_best(bv, bp >= 0, bp);
+    const int act = W - j;  // unfinished columns
+    auto put_row = [&](T* dst) {
+#pragma unroll
+      for (int u = 0; u < RPT; u++)
+        if (RPT == 1 || bu == u) {
+#pragma unroll
+          for (int i = 0; i < W; i += V) {
+            if (i < act) {
+              int4 q;
+              memcpy(&q, &v[u][i], 16);
+              *reinterpret_cast<int4*>(dst + i) = q;
+            }
+          }
+        }
+    };
+    if (lane == max(wl, 0)) {
+      sh.key[buf][warp] = bv;
+      sh.pos[buf][warp] = wl < 0 ? -1 : bp;
+      if constexpr (XP == kGrid) put_row(sh.row[buf][warp]);
+    }
     if (XP == kCluster && tid == 0)
-      mbar_arrive_expect_tx(&sh.bar[buf], (unsigned)(G * (W * sizeof(T) + 16)));
+      mbar_arrive_expect_tx(&sh.bar[buf], (unsigned)(G * (((act + V - 1) / V) * 16 + 16)));
     __syncthreads();
-    int p;
-    const T* pr;
+    int cw = -1;  // the warp with the best row (grid: known to warp 0 only)
     if (XP != kGrid || warp == 0) {
       const T ck = lane < NW ? sh.key[buf][lane] : T(0);
       const int cp = lane < NW ? sh.pos[buf][lane] : -1;
-      const int cw = warp_best(ck, cp >= 0, cp);
-      const int cwi = max(cw, 0);
-      if constexpr (XP == kSingle) {
-        p = cw >= 0 ? sh.pos[buf][cwi] : -1;
-        pr = sh.row[buf][cwi];
-      } else {
-        const T kv = sh.key[buf][cwi];
-        const int kp = cw >= 0 ? sh.pos[buf][cwi] : -1;
-        unsigned k0, k1;
-        key_words(kv, k0, k1);
-        if constexpr (XP == kCluster) {
-          // lanes 0 .. W/V-1 carry the row, the next one the header
-          constexpr int NP = W / V;
-          uint4 d = make_uint4(k0, k1, (unsigned)kp, 0u);
-          if (lane < NP) d = *reinterpret_cast<const uint4*>(&sh.row[buf][cwi][lane * V]);
-          const uint32_t dst = lane < NP ? smem_u32(&sh.crow[buf][cta][lane * V]) : smem_u32(&sh.chdr[buf][cta]);
-          const uint32_t bar = smem_u32(&sh.bar[buf]);
-          for (int q = warp; q < G; q += NW)
-            if (lane <= NP) st_async16(dst, bar, q, d);
-          if (!dead) {
-            long long n = 0;
-            while (!mbar_try_wait(&sh.bar[buf], (j >> 1) & 1)) {
-              if (++n > a.spin) {
-                dev_fail(a.st, LU_ERR_TIMEOUT, 201);
-                dead = true;
-                break;
-              }
-            }
+      cw = warp_best(ck, cp >= 0, cp);
+    }
+    if (XP != kGrid && warp == cw && lane == wl) put_row(sh.urow[j]);
+    const T* pr;
+    bool none;
+    [[maybe_unused]] int chosen = -1, chosen_lane = 0;  // cluster: the chosen position, in a lane
+    if constexpr (XP == kSingle) {
+      __syncthreads();
+      none = cw < 0;
+      pr = sh.urow[j];
+      if (tid == 0) sh.p[j] = none ? -1 : sh.pos[buf][cw];
+    } else if constexpr (XP == kCluster) {
+      __syncthreads();  // the row is in shared memory: each warp sends it to its share of the peers
+      // lanes 0 .. np-1 carry the row, the next one the header
+      const int np = (act + V - 1) / V;
+      unsigned k0, k1;
+      key_words(sh.key[buf][max(cw, 0)], k0, k1);
+      uint4 d = make_uint4(k0, k1, (unsigned)(cw >= 0 ? sh.pos[buf][cw] : -1), 0u);
+      if (lane < np) d = *reinterpret_cast<const uint4*>(&sh.urow[j][lane * V]);
+      const uint32_t dst = lane < np ? smem_u32(&sh.crow[buf][cta][lane * V]) : smem_u32(&sh.chdr[buf][cta]);
+      const uint32_t bar = smem_u32(&sh.bar[buf]);
+      if (lane <= np)
+        for (int q = warp; q < G; q += NW) st_async16(dst, bar, q, d);
+      if (!dead) {
+        long long n = 0;
+        while (!mbar_try_wait(&sh.bar[buf], (j >> 1) & 1)) {
+          if (++n > a.spin) {
+            dev_fail(a.st, LU_ERR_TIMEOUT, 201);
+            dead = true;
+            break;
           }
-          __syncwarp();
-          const uint4 hd = sh.chdr[buf][lane & (kMaxCluster - 1)];
-          T hv;
-          key_value(hd.x, hd.y, hv);
-          const int hp = lane < G ? (int)hd.z : -1;
-          const int q = warp_best(hv, hp >= 0, hp);
-          p = q >= 0 ? __shfl_sync(0xffffffffu, hp, q) : -1;
-          pr = sh.crow[buf][max(q, 0)];
-        } else {
-          // ---- publish header and row, read every CTA's header
-          constexpr int NP = (NWORDS + 2) / 3;
-          const unsigned tag = a.tag0 + (unsigned)j + 1u;
-          ulonglong2* hdr = a.pkt + (size_t)buf * kMaxLeafCTAs;
-          ulonglong2* rows = a.pkt + 2 * kMaxLeafCTAs + (size_t)buf * kMaxLeafCTAs * kLeafRowPackets;
-          const unsigned* w = reinterpret_cast<const unsigned*>(sh.row[buf][cwi]);
-          unsigned w0 = k0, w1 = k1, w2 = (unsigned)kp;
-          if (lane < NP) {
-            w0 = w[3 * lane];
-            w1 = 3 * lane + 1 < NWORDS ? w[3 * lane + 1] : 0u;
-            w2 = 3 * lane + 2 < NWORDS ? w[3 * lane + 2] : 0u;
-          }
-          if (lane <= NP) st_packet(lane < NP ? rows + cta * kLeafRowPackets + lane : hdr + cta, w0, w1, w2, tag);
-          constexpr int E = (kMaxLeafCTAs + 31) / 32;
-          uint4 h[E];
-          long long polls = 0;
-          int bad = 0;
-          for (;;) {
-            bool ok = true;
-#pragma unroll
-            for (int e = 0; e < E; e++)
-              if (lane + 32 * e < G) h[e] = ld_packet(hdr + lane + 32 * e);
-#pragma unroll
-            for (int e = 0; e < E; e++)
-              if (lane + 32 * e < G) ok = ok && h[e].w == tag;
-            if (__all_sync(0xffffffffu, ok)) break;
-            bool stop = ++polls > a.spin;
-            if ((polls & 255) == 0 && ld_acquire_s32(&a.st->code) != 0) stop = true;
-            if (__any_sync(0xffffffffu, stop)) { bad = 1; break; }
-          }
-          T bv = 0;
-          int bp = -1, bq = 0;
-#pragma unroll
-          for (int e = 0; e < E; e++) {
-            if (lane + 32 * e < G) {
-              T x;
-              key_value(h[e].x, h[e].y, x);
-              const int ps = (int)h[e].z;
-              if (ps >= 0 && (x > bv || (x == bv && bp >= 0 && ps < bp))) {
-                bv = x;
-                bp = ps;
-                bq = lane + 32 * e;
-              }
-            }
-          }
-          const int wl = warp_best(bv, bp >= 0, bp);
-          p = -1;
-          if (wl >= 0 && !bad) {
-            const int q = __shfl_sync(0xffffffffu, bq, wl);
-            p = __shfl_sync(0xffffffffu, bp, wl);
-            uint4 d;
-            for (polls = 0;;) {
-              bool ok = true;
-              if (lane < NP) {
-                d = ld_packet(rows + q * kLeafRowPackets + lane);
-                ok = d.w == tag;
-              }
-              if (__all_sync(0xffffffffu, ok)) break;
-              if (__any_sync(0xffffffffu, ++polls > a.spin)) { bad = 1; break; }
-            }
-            unsigned* dst = reinterpret_cast<unsigned*>(sh.urow[j]);
-            if (lane < NP) {
-              dst[3 * lane] = d.x;
-              if (3 * lane + 1 < NWORDS) dst[3 * lane + 1] = d.y;
-              if (3 * lane + 2 < NWORDS) dst[3 * lane + 2] = d.z;
-            }
-          }
-          if (bad && lane == 0) dev_fail(a.st, LU_ERR_TIMEOUT, 201);
-          if (lane == 0) sh.p[j] = bad ? -2 : p;
         }
       }
-    }
-    if constexpr (XP == kGrid) {
+      __syncwarp();
+      const uint4 hd = sh.chdr[buf][lane & (kMaxCluster - 1)];
+      T hv;
+      key_value(hd.x, hd.y, hv);
+      const int hp = lane < G ? (int)hd.z : -1;
+      const int q = warp_best(hv, hp >= 0, hp);
+      none = q < 0;
+      chosen = hp;
+      chosen_lane = max(q, 0);
+      pr = sh.crow[buf][max(q, 0)];
+      if (warp == 0 && lane == max(q, 0)) sh.p[j] = none ? -1 : hp;
+    } else {
+      const unsigned tag = a.tag0 + (unsigned)j + 1u;
+      ulonglong2* hdr = a.pkt + (size_t)buf * kMaxLeafCTAs;
+      ulonglong2* rows = a.pkt + 2 * kMaxLeafCTAs + (size_t)buf * kMaxLeafCTAs * kLeafRowPackets;
+      if (warp == 0) {
+        // ---- publish header and row
+        const int np = (act * WPT + 2) / 3;  // packets of the row's unfinished part
+        unsigned w0, w1, w2 = (unsigned)(cw >= 0 ? sh.pos[buf][cw] : -1);
+        key_words(sh.key[buf][max(cw, 0)], w0, w1);
+        if (lane < np) {
+          const unsigned* w = reinterpret_cast<const unsigned*>(sh.row[buf][max(cw, 0)]);
+          w0 = w[3 * lane];
+          w1 = 3 * lane + 1 < NWORDS ? w[3 * lane + 1] : 0u;
+          w2 = 3 * lane + 2 < NWORDS ? w[3 * lane + 2] : 0u;
+        }
+        if (lane <= np) st_packet(lane < np ? rows + cta * kLeafRowPackets + lane : hdr + cta, w0, w1, w2, tag);
+        // ---- every CTA's header, then the best one's row
+        constexpr int E = (kMaxLeafCTAs + 31) / 32;
+        uint4 h[E];
+        long long polls = 0;
+        int bad = 0;
+        for (;;) {
+          bool ok = true;
+#pragma unroll
+          for (int e = 0; e < E; e++)
+            if (lane + 32 * e < G) h[e] = ld_packet(hdr + lane + 32 * e);
+#pragma unroll
+          for (int e = 0; e < E; e++)
+            if (lane + 32 * e < G) ok = ok && h[e].w == tag;
+          if (__all_sync(0xffffffffu, ok)) break;
+          bool stop = ++polls > a.spin;
+          if ((polls & 255) == 0 && ld_acquire_s32(&a.st->code) != 0) stop = true;
+          if (__any_sync(0xffffffffu, stop)) { bad = 1; break; }
+        }
+        T gv = 0;
+        int gp = -1, gq = 0;
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+          if (lane + 32 * e < G) {
+            T x;
+            key_value(h[e].x, h[e].y, x);
+            const int ps = (int)h[e].z;
+            if (ps >= 0 && (x > gv || (x == gv && gp >= 0 && ps < gp))) {
+              gv = x;
+              gp = ps;
+              gq = lane + 32 * e;
+            }
+          }
+        }
+        const int gl = warp_best(gv, gp >= 0, gp);
+        int p = -1;
+        if (gl >= 0 && !bad) {
+          const int q = __shfl_sync(0xffffffffu, gq, gl);
+          p = __shfl_sync(0xffffffffu, gp, gl);
+          uint4 d;
+          for (polls = 0;;) {
+            bool ok = true;
+            if (lane < np) {
+              d = ld_packet(rows + q * kLeafRowPackets + lane);
+              ok = d.w == tag;
+            }
+            if (__all_sync(0xffffffffu, ok)) break;
+            if (__any_sync(0xffffffffu, ++polls > a.spin)) { bad = 1; break; }
+          }
+          unsigned* dst = reinterpret_cast<unsigned*>(sh.urow[j]);
+          if (lane < np) {
+            dst[3 * lane] = d.x;
+            if (3 * lane + 1 < NWORDS) dst[3 * lane + 1] = d.y;
+            if (3 * lane + 2 < NWORDS) dst[3 * lane + 2] = d.z;
+          }
+        }
+        if (bad && lane == 0) dev_fail(a.st, LU_ERR_TIMEOUT, 201);
+        if (lane == 0) sh.p[j] = bad ? -2 : p;
+      }
       __syncthreads();
-      p = sh.p[j];
+      const int p = sh.p[j];
       if (p == -2) return;
+      none = p < 0;
       pr = sh.urow[j];
-    } else if (warp == (j & (NW - 1))) {  // keep the chosen row; one warp of eight in turn
-      if (p >= 0)
-        for (int k = lane; k < W; k += 32) sh.urow[j][k] = pr[k];
-      if (lane == 0) sh.p[j] = p;
     }
 
     // ---- rename, multipliers (true division), rank-1 update, rotation.  No
     //      usable pivot: the row at j stays, nothing is scaled or updated
-    const bool none = p < 0;
+    int pj = j;
     if (none) {
       pr = sh.zero;
 #pragma unroll
@@ -388,8 +404,13 @@ __global__ void __launch_bounds__(NT, 1) getf2_leaf_kernel(T* P, T* prow0, LeafA
           for (int i = 0; i < W; i++) sh.urow[j][i] = v[u][i];
         }
     }
-    const int pj = none ? j : p;
     const T piv = pr[0];
+    if (!none) {
+      if constexpr (XP == kSingle) pj = sh.pos[buf][cw];
+      else if constexpr (XP == kGrid) pj = sh.p[j];
+      else pj = __shfl_sync(0xffffffffu, chosen, chosen_lane);
+    }
+    if (tid == 0) sh.piv[j] = piv;
     T m[RPT];
 #pragma unroll
     for (int u = 0; u < RPT; u++) {
@@ -440,7 +461,7 @@ __global__ void __launch_bounds__(NT, 1) getf2_leaf_kernel(T* P, T* prow0, LeafA
   if (cta == 0 && tid < ncols) {
     const int p = sh.p[tid];
     a.ipiv[tid] = a.row_base + (p < 0 ? tid : p);
-    if (p >= 0 && !(fabs((double)sh.urow[tid][0]) > a.thr)) dev_singular(a.st, a.info_base + tid + 1);
+    if (p >= 0 && !(fabs((double)sh.piv[tid]) > a.thr)) dev_singular(a.st, a.info_base + tid + 1);
   }
 
   // ---- the interchanges on the enclosing panel's other columns
