@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <algorithm>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -29,6 +30,23 @@ struct MatF64 {
 };
 
 int ensure_kernels_init();
+
+// What destroyed handles leave for the next ones, per device (pool.cu): device
+// blocks, and streams, events and a pinned word.  A program that makes a handle
+// per call (autograd does) otherwise spends 2 - 11 ms in some twenty
+// allocations and frees, each of which may wait for the device.  Bounded (1/64
+// of the device's memory, 8 sets of streams), given back when an allocation
+// fails or after 32 destroys without use; every function locks.
+struct HandleRes {
+  cudaStream_t sP = nullptr, sG = nullptr;  // sP: highest priority
+  cudaEvent_t ev[6] = {};                   // timing disabled
+  void* pinned = nullptr;                   // sizeof(ResidualAccum)
+};
+int pool_alloc(void** p, size_t bytes, size_t* got);
+// p must not be in use by the device any more
+void pool_free(int device, void* p, size_t bytes);
+int pool_take_res(HandleRes* r);
+void pool_give_res(int device, const HandleRes& r);
 
 }  // namespace lub
 
@@ -155,7 +173,8 @@ struct lu_handle_s {
   int res_rows = 0;
   size_t resident_cap = ~size_t(0);
   int64_t host_copied = 0;  // bytes of host A copied to the device, running total
-  std::vector<void*> allocs;
+  std::vector<std::pair<void*, size_t>> allocs;  // block, its size in the pool
+  lub::HandleRes res;
   size_t bytes = 0;
   long long spin = 0;
   // CUDA-graph replay of factorisation schedules (cfg.use_graph)
@@ -198,11 +217,9 @@ struct lu_handle_s {
   template <typename T>
   int alloc(T** p, size_t count) {
     void* q = nullptr;
-    if (cudaMalloc(&q, std::max<size_t>(count * sizeof(T), 16)) != cudaSuccess) {
-      cudaGetLastError();
-      return LU_ERR_NOMEM;
-    }
-    allocs.push_back(q);
+    size_t got = 0;
+    if (int rc = lub::pool_alloc(&q, count * sizeof(T), &got)) return rc;
+    allocs.emplace_back(q, got);
     bytes += count * sizeof(T);
     *p = static_cast<T*>(q);
     return LU_OK;
@@ -210,7 +227,8 @@ struct lu_handle_s {
   void release(void* p) {
     if (!p) return;
     cudaFree(p);
-    allocs.erase(std::remove(allocs.begin(), allocs.end(), p), allocs.end());
+    allocs.erase(std::remove_if(allocs.begin(), allocs.end(), [p](const auto& a) { return a.first == p; }),
+                 allocs.end());
   }
   size_t clear_bytes() const { return sizeof(ulonglong2) * lub::kLeafPackets + sizeof(unsigned) * n_counters; }
   unsigned* take_counter() {

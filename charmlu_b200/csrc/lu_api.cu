@@ -329,15 +329,16 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
     int lo = 0, hi = 0;
     cudaDeviceGetStreamPriorityRange(&lo, &hi);
     h->prio_hi = hi;
-    if (cudaStreamCreateWithPriority(&h->sP, cudaStreamNonBlocking, hi) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->evFork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->evP, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->evN, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->evR, cudaEventDisableTiming) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&h->sG, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->evG0, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->evG1, cudaEventDisableTiming) != cudaSuccess)
-      s = LU_ERR_CUDA;
+    s = pool_take_res(&h->res);
+    h->sP = h->res.sP;
+    h->sG = h->res.sG;
+    h->evFork = h->res.ev[0];
+    h->evP = h->res.ev[1];
+    h->evN = h->res.ev[2];
+    h->evR = h->res.ev[3];
+    h->evG0 = h->res.ev[4];
+    h->evG1 = h->res.ev[5];
+    h->racc_host = static_cast<ResidualAccum*>(h->res.pinned);
   }
   h->leaf_ctas = h->num_sms;
   h->gemm_ctas = h->num_sms;
@@ -368,7 +369,6 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
   if (s == LU_OK) s = h->alloc(&h->vec, n);
   if (s == LU_OK) s = h->alloc(&h->vec2, n);
   if (s == LU_OK) s = h->alloc(&h->racc, 1);
-  if (s == LU_OK && cudaMallocHost(&h->racc_host, sizeof(ResidualAccum)) != cudaSuccess) s = LU_ERR_NOMEM;
   if (s == LU_OK && cudaMemset(h->st, 0, sizeof(DevStatus)) != cudaSuccess) s = LU_ERR_CUDA;
   if (s != LU_OK) {
     lu_destroy(h);
@@ -381,23 +381,28 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
 int lu_destroy(lu_handle h) {
   if (!h) return LU_ERR_ARG;
   for (cudaEvent_t e : h->pool) cudaEventDestroy(e);
-  if (h->evFork) cudaEventDestroy(h->evFork);
-  if (h->evP) cudaEventDestroy(h->evP);
-  if (h->evN) cudaEventDestroy(h->evN);
-  if (h->evR) cudaEventDestroy(h->evR);
-  if (h->sP) cudaStreamDestroy(h->sP);
   for (auto& g : h->gslot)
     if (g.exec) cudaGraphExecDestroy(g.exec);
-  if (h->evG0) cudaEventDestroy(h->evG0);
-  if (h->evG1) cudaEventDestroy(h->evG1);
-  if (h->sG) cudaStreamDestroy(h->sG);
   for (int b = 0; b < 2; b++) {
     if (h->evReady[b]) cudaEventDestroy(h->evReady[b]);
     if (h->evFree[b]) cudaEventDestroy(h->evFree[b]);
   }
   if (h->sCopy) cudaStreamDestroy(h->sCopy);
-  for (void* p : h->allocs) cudaFree(p);
-  if (h->racc_host) cudaFreeHost(h->racc_host);
+  // the handle's work may still run: wait as the frees would, on its device
+  int cur = h->device;
+  cudaGetDevice(&cur);
+  if (cur != h->device) cudaSetDevice(h->device);
+  const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+  if (!idle) cudaGetLastError();
+  for (auto& blk : h->allocs) {
+    if (idle) pool_free(h->device, blk.first, blk.second);
+    else cudaFree(blk.first);
+  }
+  if (h->res.sP) {
+    if (idle) pool_give_res(h->device, h->res);
+    else pool_give_res(-1, h->res);
+  }
+  if (cur != h->device) cudaSetDevice(cur);
   delete h;
   return LU_OK;
 }
@@ -442,8 +447,7 @@ int lu_transpose_square(double* dA, int64_t n, int64_t lda, void* stream) {
 static int ensure_tmpB(lu_handle h, size_t elems) {
   if (h->tmpB_elems >= elems) return LU_OK;
   if (h->tmpB) {
-    cudaFree(h->tmpB);
-    h->allocs.erase(std::remove(h->allocs.begin(), h->allocs.end(), (void*)h->tmpB), h->allocs.end());
+    h->release(h->tmpB);
     h->tmpB = nullptr;
   }
   LUB_TRY(h->alloc(&h->tmpB, elems));

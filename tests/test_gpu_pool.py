@@ -1,0 +1,66 @@
+"""Handles made from what earlier ones left (device blocks, streams, events):
+blocks with another order's leftovers, several threads and streams at once."""
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _system(n, seed):
+    rng = np.random.default_rng(seed)
+    A = rng.uniform(-0.5, 0.5, (n, n)) + np.eye(n) * np.sqrt(n)
+    b = rng.uniform(-0.5, 0.5, n)
+    buf = torch.zeros(n, n + (n & 1), dtype=torch.float64, device="cuda")[:, :n]
+    buf.copy_(torch.from_numpy(A))
+    return buf, torch.from_numpy(b).cuda(), np.linalg.solve(A, b)
+
+
+def test_reused_blocks_of_another_order(cuda_dev):
+    import charmlu_b200 as lu
+    orders = [900, 333, 1024, 901, 334, 900]
+    for it in range(2):
+        for n in orders:
+            A, b, ref = _system(n, n)
+            for prec in (lu.LU_PREC_FP16X3, lu.LU_PREC_FP64):
+                s = lu.LUSolver(lu.LUConfig(n, 64, precision=prec, lookahead=bool(it), use_graph=bool(n & 1),
+                                            ir_target=1e-3))
+                if prec == lu.LU_PREC_FP64:
+                    W, x = A.clone() if n % 2 == 0 else torch.nn.functional.pad(A, (0, 1))[:, :n], b.clone()
+                    s.factor_solve(W, x)
+                    assert s.status() == 0
+                else:
+                    x, info = s.refine_solve(A, b)
+                    assert info["status"] == 0
+                # well conditioned (kappa < 10): a backward stable solution is this close
+                assert np.abs(x.cpu().numpy() - ref).max() <= 1e-11 * np.abs(ref).max(), (n, prec)
+                s.close()
+
+
+def test_threads_with_their_own_streams(cuda_dev):
+    import charmlu_b200 as lu
+    bad = []
+
+    def work(k):
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                for it in range(6):
+                    n = 256 + 32 * ((k + it) % 5)
+                    A, b, ref = _system(n, 10 * k + it)
+                    s = lu.LUSolver(lu.LUConfig(n, 64))
+                    s.factor_solve(A, b, stream=stream)
+                    if s.status(stream) != 0 or np.abs(b.cpu().numpy() - ref).max() > 1e-11 * np.abs(ref).max():
+                        bad.append((k, it))
+                    s.close()
+        except Exception as e:  # reported by the main thread
+            bad.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
