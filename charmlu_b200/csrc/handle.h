@@ -110,8 +110,7 @@ struct lu_handle_s {
   int32_t* perm = nullptr;
   int32_t* perm_work = nullptr;
   int32_t* perm_lists = nullptr;  // composed pivot batches (ipiv -> perm)
-  int* trsv_flags = nullptr;
-  unsigned* trsv_ticket = nullptr;
+  int* trsv_flags = nullptr;   // kPipeScratchInts: the substitution pipelines' counters and packets
   double* vec = nullptr;
   double* vec2 = nullptr;
   double* tmpB = nullptr;      // n x nrhs staging block of multi-RHS solves (grown on demand)

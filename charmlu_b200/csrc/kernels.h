@@ -109,16 +109,22 @@ int launch_trsm_llu_block(const float* L, int64_t ldl, float* B, int64_t ldb, in
 // B (w x ncols) <- L^{-1} B, L unit lower, w <= 512, FP32; dinv: 16 x 1024 floats of scratch
 int launch_trsm_wide(const float* L, int64_t ldl, float* B, int64_t ldb, int w, int ncols, float* dinv,
                      cudaStream_t s);
-// single/multi right-hand side substitution with flags (persistent tickets)
+// Scratch of the substitution pipelines (flags, 16-byte aligned): progress and
+// ticket counters, then a ring of 4 blocks' rows as tagged 16-byte packets
+// (64 rows, or 64 x 16); cleared by each launch
+constexpr int kPipeRing = 4;
+constexpr int kTrsvScratchInts = 8 + kPipeRing * 64 * 4;
+constexpr int kPipeScratchInts = 8 + kPipeRing * 64 * 16 * 4;
+// single/multi right-hand side substitution (persistent tickets)
 template <typename T>
-int launch_trsv(const T* LU, int64_t lda, int n, T* x, int upper, int* flags, unsigned* ticket, DevStatus* st,
+int launch_trsv(const T* LU, int64_t lda, int n, T* x, int upper, int* flags, DevStatus* st,
                 long long spin, cudaStream_t s);
 
 // multi-RHS pipelined triangular solve (mode 0 L, 1 U, 2 U^T, 3 L^T) on a
 // row-major n x nrhs FP64 block; factors stored as TS (double or float)
 template <typename TS>
 int launch_trsm_pipe(const TS* LU, int64_t lda, int n, double* Y, int64_t ldy, int nrhs, int mode, int* flags,
-                     unsigned* ticket, DevStatus* st, long long spin, cudaStream_t s);
+                     DevStatus* st, long long spin, cudaStream_t s);
 
 // ---- multi-RHS refinement (up to 16 columns, ld 16 work blocks)
 constexpr int kMultiMaxSplits = 16;  // reduction splits of the residual product
@@ -162,7 +168,7 @@ int launch_residual_f64_rows(const double* Arows, int64_t lda, int rows, int row
                              const double* b, double* r, ResidualAccum* acc, cudaStream_t s);
 // factors stored as TS, vector and arithmetic in T (FP32 factors, FP64 vector)
 template <typename TS, typename T>
-int launch_trsv_mixed(const TS* LU, int64_t lda, int n, T* x, int upper, int* flags, unsigned* ticket, DevStatus* st,
+int launch_trsv_mixed(const TS* LU, int64_t lda, int n, T* x, int upper, int* flags, DevStatus* st,
                       long long spin, cudaStream_t s);
 // y[i] = v[perm[i]] * scale (scale = 1/||r||inf from acc when acc is given)
 int launch_gather_f64(const double* v, const int32_t* perm, double* y, int n, double scale, const ResidualAccum* acc,

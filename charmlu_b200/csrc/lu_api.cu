@@ -255,8 +255,8 @@ int factor_f64_schedule(lu_handle h, double* dA, int64_t lda, int32_t* ipiv, dou
 int solve_permuted_f64(lu_handle h, const double* LU, int64_t lda, double* x, cudaStream_t s) {
   const int n = (int)h->cfg.n;
   Prof pf(h, s, LU_PH_SOLVE, 2.0 * n * (double)n);
-  LUB_TRY(launch_trsv<double>(LU, lda, n, x, 0, h->trsv_flags, h->trsv_ticket, h->st, h->spin, s));
-  LUB_TRY(launch_trsv<double>(LU, lda, n, x, 1, h->trsv_flags, h->trsv_ticket, h->st, h->spin, s));
+  LUB_TRY(launch_trsv<double>(LU, lda, n, x, 0, h->trsv_flags, h->st, h->spin, s));
+  LUB_TRY(launch_trsv<double>(LU, lda, n, x, 1, h->trsv_flags, h->st, h->spin, s));
   return LU_OK;
 }
 
@@ -290,7 +290,7 @@ size_t lu_workspace_bytes(const lu_config* cfg) {
   b += sizeof(ulonglong2) * kLeafPackets;
   b += 2 * sizeof(int32_t) * (4 * kMaxBatch + 1);
   b += sizeof(int32_t) * 2 * n;
-  b += sizeof(int) * (n / 64 + 2) + sizeof(unsigned);
+  b += sizeof(int) * kPipeScratchInts;
   b += sizeof(double) * 2 * n;
   b += sizeof(ResidualAccum);
   return b;
@@ -364,8 +364,7 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
   if (s == LU_OK) s = h->alloc(&h->perm, n);
   if (s == LU_OK) s = h->alloc(&h->perm_work, n);
   if (s == LU_OK) s = h->alloc(&h->perm_lists, lub::ipiv_to_perm_work_ints((int)n));
-  if (s == LU_OK) s = h->alloc(&h->trsv_flags, n / 64 + 2);
-  if (s == LU_OK) s = h->alloc(&h->trsv_ticket, 1);
+  if (s == LU_OK) s = h->alloc(&h->trsv_flags, kPipeScratchInts);
   if (s == LU_OK) s = h->alloc(&h->vec, n);
   if (s == LU_OK) s = h->alloc(&h->vec2, n);
   if (s == LU_OK) s = h->alloc(&h->racc, 1);
@@ -464,8 +463,8 @@ static int solve_trans_multi(lu_handle h, const double* dLU, int64_t lda, const 
   LUB_CUDA(cudaMemcpy2DAsync(h->tmpB, sizeof(double) * nrhs, B, sizeof(double) * ldb, sizeof(double) * nrhs, n,
                              cudaMemcpyDeviceToDevice, s));
   Prof pf(h, s, LU_PH_SOLVE, 2.0 * n * (double)n * nrhs);
-  LUB_TRY(launch_trsm_pipe(dLU, lda, n, h->tmpB, nrhs, nrhs, 2, h->trsv_flags, h->trsv_ticket, h->st, h->spin, s));
-  LUB_TRY(launch_trsm_pipe(dLU, lda, n, h->tmpB, nrhs, nrhs, 3, h->trsv_flags, h->trsv_ticket, h->st, h->spin, s));
+  LUB_TRY(launch_trsm_pipe(dLU, lda, n, h->tmpB, nrhs, nrhs, 2, h->trsv_flags, h->st, h->spin, s));
+  LUB_TRY(launch_trsm_pipe(dLU, lda, n, h->tmpB, nrhs, nrhs, 3, h->trsv_flags, h->st, h->spin, s));
   return launch_permute_rows(h->tmpB, nrhs, Y, ldy, h->perm_work, n, nrhs, 1, s);
 }
 
@@ -489,9 +488,9 @@ int lu_solve(lu_handle h, const double* dLU, int64_t lda, const int32_t* ipiv, d
   LUB_TRY(launch_permute_rows(dB, ldb, h->tmpB, nrhs, h->perm_work, n, (int)nrhs, 0, s));
   {
     Prof pf(h, s, LU_PH_SOLVE, 2.0 * n * (double)n * nrhs);
-    LUB_TRY(launch_trsm_pipe(dLU, lda, n, h->tmpB, nrhs, (int)nrhs, 0, h->trsv_flags, h->trsv_ticket, h->st,
+    LUB_TRY(launch_trsm_pipe(dLU, lda, n, h->tmpB, nrhs, (int)nrhs, 0, h->trsv_flags, h->st,
                              h->spin, s));
-    LUB_TRY(launch_trsm_pipe(dLU, lda, n, h->tmpB, nrhs, (int)nrhs, 1, h->trsv_flags, h->trsv_ticket, h->st,
+    LUB_TRY(launch_trsm_pipe(dLU, lda, n, h->tmpB, nrhs, (int)nrhs, 1, h->trsv_flags, h->st,
                              h->spin, s));
   }
   LUB_CUDA(cudaMemcpy2DAsync(dB, sizeof(double) * ldb, h->tmpB, sizeof(double) * nrhs, sizeof(double) * nrhs, n,
@@ -737,7 +736,7 @@ int lu_trsv_block(lu_handle h, const double* dT, int64_t ldt, int32_t w, int32_t
   LUB_TRY(ensure_kernels_init());
   cudaStream_t s = (cudaStream_t)stream;
   Prof pf(h, s, LU_PH_SOLVE, (double)w * w);
-  return launch_trsv<double>(dT, ldt, w, dx, upper ? 1 : 0, h->trsv_flags, h->trsv_ticket, h->st, h->spin, s);
+  return launch_trsv<double>(dT, ldt, w, dx, upper ? 1 : 0, h->trsv_flags, h->st, h->spin, s);
 }
 
 int lu_copy_2d(void* dst, int64_t dpitch, const void* src, int64_t spitch, int64_t width, int64_t rows,

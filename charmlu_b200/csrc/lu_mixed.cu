@@ -467,17 +467,17 @@ int factor_mixed(lu_handle h, cudaStream_t s, const double* rest_src, int64_t re
 int solve32(lu_handle h, float* v, cudaStream_t s) {
   const int n = (int)h->cfg.n;
   Prof pf(h, s, LU_PH_SOLVE, 2.0 * n * (double)n);
-  LUB_TRY(launch_trsv<float>(h->A32, h->ld32, n, v, 0, h->trsv_flags, h->trsv_ticket, h->st, h->spin, s));
-  return launch_trsv<float>(h->A32, h->ld32, n, v, 1, h->trsv_flags, h->trsv_ticket, h->st, h->spin, s);
+  LUB_TRY(launch_trsv<float>(h->A32, h->ld32, n, v, 0, h->trsv_flags, h->st, h->spin, s));
+  return launch_trsv<float>(h->A32, h->ld32, n, v, 1, h->trsv_flags, h->st, h->spin, s);
 }
 
 // M^{-1} v in working precision: FP32 factors, FP64 vector and arithmetic
 int solve_f32_factors_f64(lu_handle h, double* v, cudaStream_t s) {
   const int n = (int)h->cfg.n;
   Prof pf(h, s, LU_PH_SOLVE, 2.0 * n * (double)n);
-  LUB_TRY((launch_trsv_mixed<float, double>(h->A32, h->ld32, n, v, 0, h->trsv_flags, h->trsv_ticket, h->st,
+  LUB_TRY((launch_trsv_mixed<float, double>(h->A32, h->ld32, n, v, 0, h->trsv_flags, h->st,
                                              h->spin, s)));
-  return launch_trsv_mixed<float, double>(h->A32, h->ld32, n, v, 1, h->trsv_flags, h->trsv_ticket, h->st, h->spin,
+  return launch_trsv_mixed<float, double>(h->A32, h->ld32, n, v, 1, h->trsv_flags, h->st, h->spin,
                                            s);
 }
 
@@ -873,9 +873,9 @@ int prec_trans_vec(lu_handle h, double* v, double* tmp, cudaStream_t s) {
   const int n = (int)h->cfg.n;
   Prof pf(h, s, LU_PH_SOLVE, 2.0 * n * (double)n);
   LUB_CUDA(cudaMemcpyAsync(tmp, v, sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
-  LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, tmp, 1, 1, 2, h->trsv_flags, h->trsv_ticket, h->st, h->spin,
+  LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, tmp, 1, 1, 2, h->trsv_flags, h->st, h->spin,
                                   s));
-  LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, tmp, 1, 1, 3, h->trsv_flags, h->trsv_ticket, h->st, h->spin,
+  LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, tmp, 1, 1, 3, h->trsv_flags, h->st, h->spin,
                                   s));
   return launch_vec_scatter(tmp, h->perm32, v, n, s);
 }
@@ -921,15 +921,15 @@ int multi_correction(lu_handle h, int trans, int k, cudaStream_t s) {
   Prof pf(h, s, LU_PH_SOLVE, 2.0 * n * (double)n * k);
   if (!trans) {
     LUB_TRY(launch_permute_rows(h->mr_R, 16, h->mr_D, 16, h->perm32, n, k, 0, s));
-    LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, h->mr_D, 16, k, 0, h->trsv_flags, h->trsv_ticket, h->st,
+    LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, h->mr_D, 16, k, 0, h->trsv_flags, h->st,
                                     h->spin, s));
-    LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, h->mr_D, 16, k, 1, h->trsv_flags, h->trsv_ticket, h->st,
+    LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, h->mr_D, 16, k, 1, h->trsv_flags, h->st,
                                     h->spin, s));
     return launch_multi_add(h->mr_X, h->mr_D, h->perm32, n, k, 0, s);
   }
-  LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, h->mr_R, 16, k, 2, h->trsv_flags, h->trsv_ticket, h->st,
+  LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, h->mr_R, 16, k, 2, h->trsv_flags, h->st,
                                   h->spin, s));
-  LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, h->mr_R, 16, k, 3, h->trsv_flags, h->trsv_ticket, h->st,
+  LUB_TRY(launch_trsm_pipe<float>(h->A32, h->ld32, n, h->mr_R, 16, k, 3, h->trsv_flags, h->st,
                                   h->spin, s));
   return launch_multi_add(h->mr_X, h->mr_R, h->perm32, n, k, 1, s);
 }

@@ -36,8 +36,9 @@ namespace {
 
 constexpr int kNoAllocMaxN = 1 << 17;             // largest order accepted (131072)
 constexpr int kNoAllocBlocks = kNoAllocMaxN / 64;  // 64-row substitution blocks
-// ints: [0, 4) DevStatus, [4] ticket, [8, 8 + blocks + 2) ready flags
+// ints: [0, 4) DevStatus, [8, ..) the pipeline's counters and packets
 constexpr int kNoAllocInts = 8 + kNoAllocBlocks + 2;
+static_assert(8 + kTrsvScratchInts <= kNoAllocInts, "");
 
 static __device__ __align__(256) int g_noalloc_scratch[kNoAllocInts];
 
@@ -84,14 +85,13 @@ extern "C" LU_API int lu_solve_noalloc(const double* dLU, int64_t lda, int64_t n
   int* base = nullptr;
   LUB_TRY(noalloc_scratch(&base));
   DevStatus* st = reinterpret_cast<DevStatus*>(base);
-  unsigned* ticket = reinterpret_cast<unsigned*>(base + 4);
   int* flags = base + 8;
   const long long spin = 1LL << 24;
   LUB_CUDA(cudaMemsetAsync(st, 0, sizeof(DevStatus), s));
   LUB_TRY(launch_ipiv_apply_vector(ipiv, (int)n, db, s));
-  // launch_trsv clears the flags and the ticket on the stream before each launch
-  LUB_TRY(launch_trsv<double>(dLU, lda, (int)n, db, 0, flags, ticket, st, spin, s));
-  LUB_TRY(launch_trsv<double>(dLU, lda, (int)n, db, 1, flags, ticket, st, spin, s));
+  // launch_trsv clears the counters and packets on the stream before each launch
+  LUB_TRY(launch_trsv<double>(dLU, lda, (int)n, db, 0, flags, st, spin, s));
+  LUB_TRY(launch_trsv<double>(dLU, lda, (int)n, db, 1, flags, st, spin, s));
   if (d_status) {
     noalloc_status_kernel<<<1, 1, 0, s>>>(st, d_status);
     LUB_LAUNCH_CHECK();

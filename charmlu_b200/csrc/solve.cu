@@ -386,6 +386,45 @@ __device__ __forceinline__ bool wait_progress(const int* counter, int need, int*
   return true;
 }
 
+// A finished block's rows also leave as 16-byte packets {value, tag} in a ring
+// of kPipeRing blocks, ahead of the counter (n = 8192, forward and backward:
+// one column 864 -> 608 us; 16 columns, with two chains, 840 -> 739 us): one 128-bit access each, so the
+// data is its own flag, and the next blocks read them without the publisher's
+// fence and a second trip for the rows.  A block takes its last
+// kPipeRing - 1 predecessors this way; that the ring's slot of block t - 4 is
+// free when block t publishes follows from t having waited for t - 1, which
+// had waited for t - 2 and t - 3: the only readers of that slot.
+constexpr int kPipeNear = kPipeRing - 1;
+__device__ __forceinline__ void st_value_packet(int* p, double v, int tag) {
+  const unsigned long long lo = (unsigned long long)__double_as_longlong(v), hi = (unsigned)tag;
+  asm volatile("{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p),
+               "l"(lo), "l"(hi)
+               : "memory");
+}
+__device__ __forceinline__ void st_value_packet(int* p, float v, int tag) {
+  st_value_packet(p, __hiloint2double(0, __float_as_int(v)), tag);
+}
+__device__ __forceinline__ bool ld_value_packet(const int* p, int tag, double& v) {
+  unsigned long long lo, hi;
+  asm volatile("{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
+               : "=l"(lo), "=l"(hi)
+               : "l"(p)
+               : "memory");
+  v = __longlong_as_double((long long)lo);
+  return (int)(unsigned)hi == tag;
+}
+__device__ __forceinline__ bool ld_value_packet(const int* p, int tag, float& v) {
+  double d;
+  const bool ok = ld_value_packet(p, tag, d);
+  v = __int_as_float(__double2loint(d));
+  return ok;
+}
+// One more unsuccessful poll: false when the wait has run out
+__device__ __forceinline__ bool keep_polling(long long& polls, DevStatus* st, long long spin, int where) {
+  if (++polls > spin) { dev_fail(st, LU_ERR_TIMEOUT, where); return false; }
+  return (polls & 255) != 0 || ld_acquire_s32(&st->code) == 0;
+}
+
 // TS: storage type of the factors; T: type of the vector and the arithmetic
 // (FP32 factors with an FP64 vector give the GMRES-IR preconditioner solve
 // in working precision at the FP32 factors' memory cost).
@@ -398,7 +437,7 @@ __host__ __device__ constexpr size_t trsv_smem() {
 
 template <typename TS, typename T, bool UPPER>
 __global__ void __launch_bounds__(256) trsv_kernel(const TS* LU, int64_t lda, int n, T* x, int* flags,
-                                                   unsigned* ticket, DevStatus* st, long long spin) {
+                                                   DevStatus* st, long long spin) {
   extern __shared__ __align__(16) unsigned char trsv_raw[];
   T* sInv = reinterpret_cast<T*>(trsv_raw);
   TS* sD = reinterpret_cast<TS*>(sInv + TB * (TB + 1));
@@ -406,7 +445,7 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TS* LU, int64_t lda, in
   __shared__ T s_rhs[TB];
   __shared__ int s_blk;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) s_blk = (int)atomicAdd(ticket, 1u);
+  if (tid == 0) s_blk = atomicAdd(&flags[1], 1);
   __syncthreads();
   const int nblk = (n + TB - 1) / TB;
   const int tk = s_blk;
@@ -476,7 +515,22 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TS* LU, int64_t lda, in
         xok[dn] = qn < seen;
         if (xok[dn]) load_x(qn, xr[dn]);
       }
-      if (q + 1 > seen) {  // block q (in ticket order) not known to be final yet
+      if (q + 1 > seen && q >= nvisit - kPipeNear) {  // a near predecessor: its packets
+        const int c = col0(q) + lane * 2;
+        const int* pk = flags + 8 + ((q & (kPipeRing - 1)) * TB + lane * 2) * 4;
+        bool got0 = c >= n, got1 = c + 1 >= n;
+        T v0 = T(0), v1 = T(0);
+        for (long long polls = 0;;) {
+          if (!got0) got0 = ld_value_packet(pk, q + 1, v0);
+          if (!got1) got1 = ld_value_packet(pk + 4, q + 1, v1);
+          if (__all_sync(0xffffffffu, got0 && got1)) break;
+          if (!__all_sync(0xffffffffu, keep_polling(polls, st, spin, 301))) { ok = false; break; }
+        }
+        if (!ok) break;
+        xr[d][0] = c < n ? v0 : T(0);
+        xr[d][1] = c + 1 < n ? v1 : T(0);
+        xok[d] = true;
+      } else if (q + 1 > seen) {  // block q (in ticket order) not known to be final yet
         int v = 0;
         if (lane == 0) ok = wait_progress(&flags[0], q + 1, &v, st, spin, 301);
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
@@ -510,7 +564,10 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TS* LU, int64_t lda, in
     }
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    if (q4 == 0 && r < rows) x[r0 + r] = sum;
+    if (q4 == 0 && r < rows) {
+      st_value_packet(flags + 8 + ((tk & (kPipeRing - 1)) * TB + r) * 4, sum, tk + 1);
+      x[r0 + r] = sum;
+    }
   }
   // CTA barrier, then thread 0's release store: the rows written above are
   // visible to every CTA that acquires the counter
@@ -528,11 +585,12 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TS* LU, int64_t lda, in
 //   MODE 3  LT: T = L^T (unit upper)     backward, tiles L[bk][bi]^T, bk > bi
 // Modes 2 and 3 are the transposed solves of the adjoint (A^T lambda = W).
 // Same ticket / progress-counter pipeline as trsv_kernel, with the inverted
-// diagonal tile.  Both 64 x 64 x 16 products of a step (an off-diagonal
-// tile against the finished rows of Y, and the inverted diagonal tile
-// against the block's right-hand side) run on the FP64 tensor pipe
-// (mma.sync m16n8k4; warp w owns output rows 16 (w / 2).., columns
-// 8 (w % 2)..).  The factor tiles do not depend on the pipeline, so they
+// diagonal tile, one chain of CTAs per 8 columns (tickets alternate between
+// the chains).  Both 64 x 64 x 8 products of a step (an off-diagonal tile
+// against the finished rows of Y, and the inverted diagonal tile against the
+// block's right-hand side) run on the FP64 tensor pipe (mma.sync m16n8k4; warp
+// w < 4 owns output rows 16 w ..).  With 16 columns in one chain each product
+// kept two warps of an SM sub-partition waiting for the pipe in turn.  The factor tiles do not depend on the pipeline, so they
 // stream through a two-stage cp.async ring (tile q+1 in flight while the
 // CTA waits for block q and applies tile q); only the 64 x 16 slice of Y
 // waits for the counter.  Tiles are read by rows in every mode (the
@@ -550,7 +608,7 @@ __host__ __device__ constexpr size_t pipe_ring_bytes() {
          sizeof(TS);
 }
 constexpr int kInvPitch = 68;
-constexpr int kYkPitch = 20;
+constexpr int kYkPitch = 12;
 template <typename TS>
 __host__ __device__ constexpr size_t pipe_smem() {
   return pipe_ring_bytes<TS>() + (size_t)TB * kInvPitch * sizeof(double);
@@ -565,8 +623,7 @@ __device__ __forceinline__ void dmma16x8x4(double (&c)[4], double a0, double a1,
 
 template <typename TS, int MODE>
 __global__ void __launch_bounds__(256, 2) trsm_pipe_kernel(const TS* LU, int64_t lda, int n, double* Y, int64_t ldy,
-                                                        int nrhs, int* flags, unsigned* ticket, DevStatus* st,
-                                                        long long spin) {
+                                                        int nrhs, int* flags, DevStatus* st, long long spin) {
   constexpr bool FWD = (MODE == 0 || MODE == 2);
   constexpr bool TRANS = (MODE >= 2);
   constexpr int TP = pipe_pitch<TS, TRANS>();
@@ -578,18 +635,24 @@ __global__ void __launch_bounds__(256, 2) trsm_pipe_kernel(const TS* LU, int64_t
   __shared__ __align__(16) double yk[TB][kYkPitch];
   __shared__ int s_blk, s_ok;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) s_blk = (int)atomicAdd(ticket, 1u);
+  if (tid == 0) s_blk = atomicAdd(&flags[1], 1);
   __syncthreads();
   const int nblk = (n + TB - 1) / TB;
-  const int tk = s_blk;
+  // ticket -> chain of 8 columns, block of it
+  const int chains = (nrhs + 7) / 8, chain = s_blk % chains, tk = s_blk / chains;
   if (tk >= nblk) return;
+  Y += 8 * chain;
+  nrhs = min(8, nrhs - 8 * chain);
+  int* progress = flags + 2 * chain;
+  int* packets = flags + 8 + chain * (kPipeRing * TB * 8 * 4);
   const int bi = FWD ? tk : nblk - 1 - tk;
   const int r0 = bi * TB, rows = min(TB, n - r0);
   const int nvisit = FWD ? bi : nblk - 1 - bi;
   // MMA fragment coordinates: group g, thread-in-group t; warp tile rows
   // m0 .. m0 + 15, columns n0 .. n0 + 7
   const int g = lane >> 2, t = lane & 3;
-  const int m0 = (warp >> 1) * 16, n0 = (warp & 1) * 8;
+  const int m0 = (warp & 3) * 16;
+  const bool mma = warp < 4;  // the other warps copy
 
   // stage a tile into ring slot `slot`: rows grow0.., cols gcol0.. (nrow x ncol valid)
   auto stage = [&](int slot, int grow0, int gcol0, int nrow, int ncol) {
@@ -616,8 +679,8 @@ __global__ void __launch_bounds__(256, 2) trsm_pipe_kernel(const TS* LU, int64_t
   double own[4];
 #pragma unroll
   for (int e = 0; e < 4; e++) {
-    const int r = m0 + g + (e >> 1) * 8, c = n0 + 2 * t + (e & 1);
-    own[e] = (r < rows && c < nrhs) ? Y[(int64_t)(r0 + r) * ldy + c] : 0.0;
+    const int r = m0 + g + (e >> 1) * 8, c = 2 * t + (e & 1);
+    own[e] = (mma && r < rows && c < nrhs) ? Y[(int64_t)(r0 + r) * ldy + c] : 0.0;
   }
   stage(0, r0, r0, rows, rows);
   asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -635,32 +698,69 @@ __global__ void __launch_bounds__(256, 2) trsm_pipe_kernel(const TS* LU, int64_t
     const int bk = FWD ? q : nblk - 1 - q;
     const int c0 = bk * TB, cw = min(TB, n - c0);
     if (q + 1 < nvisit) issue(q + 1);
-    if (q + 1 > seen) {  // block q (in ticket order) not known to be final yet
+    const bool near = q + 1 > seen && q >= nvisit - kPipeNear;
+    if (q + 1 > seen && !near) {  // block q (in ticket order) not known to be final yet
       if (tid == 0) {
         int v = 0;
-        s_ok = wait_progress(&flags[0], q + 1, &v, st, spin, 302) ? v : -1;
+        s_ok = wait_progress(progress, q + 1, &v, st, spin, 302) ? v : -1;
       }
       __syncthreads();
       seen = s_ok;
       if (seen < 0) { ok = false; break; }
     }
+    bool mine = true;  // near: this thread's rows arrived
+    if (near) {  // a near predecessor: its packets
+      // packet u of this thread: accumulator element e of lane `lane` of warp
+      // pw, in the order in which they were stored (512 bytes per store)
+      constexpr int U = TB * 8 / 256;
+      const int* pk = packets + ((q & (kPipeRing - 1)) * TB * 8) * 4;
+      double v[U];
+      unsigned todo = 0;
+      auto at = [&](int u, int& i, int& c) {
+        const int pw = (warp + 8 * u) >> 2, e = warp & 3;
+        i = pw * 16 + g + (e >> 1) * 8;
+        c = 2 * t + (e & 1);
+      };
 #pragma unroll
-    for (int u = 0; u < TB * 16 / 256; u++) {
-      const int idx = tid + u * 256;
-      const int i = idx >> 4, c = idx & 15;
-      yk[i][c] = (i < cw && c < nrhs) ? __ldcg(&Y[(int64_t)(c0 + i) * ldy + c]) : 0.0;
+      for (int u = 0; u < U; u++) {
+        int i, c;
+        at(u, i, c);
+        v[u] = 0.0;
+        if (i < cw && c < nrhs) todo |= 1u << u;
+      }
+      for (long long polls = 0; todo;) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+          if ((todo >> u) & 1u)
+            if (ld_value_packet(pk + (tid + u * 256) * 4, q + 1, v[u])) todo &= ~(1u << u);
+        if (todo && !keep_polling(polls, st, spin, 302)) { mine = false; break; }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        int i, c;
+        at(u, i, c);
+        yk[i][c] = v[u];
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < TB * 8 / 256; u++) {
+        const int idx = tid + u * 256;
+        const int i = idx >> 3, c = idx & 7;
+        yk[i][c] = (i < cw && c < nrhs) ? __ldcg(&Y[(int64_t)(c0 + i) * ldy + c]) : 0.0;
+      }
     }
     if (q + 1 < nvisit) asm volatile("cp.async.wait_group 1;" ::: "memory");
     else asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
+    if (!__syncthreads_and(mine ? 1 : 0)) { ok = false; break; }
     const TS* tq = ring + (q & 1) * TB * TP;
     // acc += T[bi][bk] * Y[bk] on this warp's 16 x 8 tile
+    if (mma)
 #pragma unroll
     for (int ks = 0; ks < TB / 4; ks++) {
       const int k = ks * 4 + t;
       const double a0 = (double)(TRANS ? tq[k * TP + m0 + g] : tq[(m0 + g) * TP + k]);
       const double a1 = (double)(TRANS ? tq[k * TP + m0 + g + 8] : tq[(m0 + g + 8) * TP + k]);
-      dmma16x8x4(acc, a0, a1, yk[k][n0 + g]);
+      dmma16x8x4(acc, a0, a1, yk[k][g]);
     }
     __syncthreads();  // ring slot, yk and s_ok are rewritten next
   }
@@ -668,25 +768,31 @@ __global__ void __launch_bounds__(256, 2) trsm_pipe_kernel(const TS* LU, int64_t
   if (!ok) return;  // uniform: every thread read the same s_ok
   // R = B_bi - off-diagonal part (into yk), then Y_bi = T^{-1} R
 #pragma unroll
-  for (int e = 0; e < 4; e++) yk[m0 + g + (e >> 1) * 8][n0 + 2 * t + (e & 1)] = own[e] - acc[e];
+  for (int e = 0; e < 4; e++)
+    if (mma) yk[m0 + g + (e >> 1) * 8][2 * t + (e & 1)] = own[e] - acc[e];
   __syncthreads();
+  if (mma) {
   double out[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
   for (int ks = 0; ks < TB / 4; ks++) {
     const int k = ks * 4 + t;
     const double a0 = TRANS ? dinv[k * kInvPitch + m0 + g] : dinv[(m0 + g) * kInvPitch + k];
     const double a1 = TRANS ? dinv[k * kInvPitch + m0 + g + 8] : dinv[(m0 + g + 8) * kInvPitch + k];
-    dmma16x8x4(out, a0, a1, yk[k][n0 + g]);
+    dmma16x8x4(out, a0, a1, yk[k][g]);
   }
 #pragma unroll
+  for (int e = 0; e < 4; e++)
+    st_value_packet(packets + ((tk & (kPipeRing - 1)) * TB * 8 + (warp * 4 + e) * 32 + lane) * 4, out[e], tk + 1);
+#pragma unroll
   for (int e = 0; e < 4; e++) {
-    const int r = m0 + g + (e >> 1) * 8, c = n0 + 2 * t + (e & 1);
+    const int r = m0 + g + (e >> 1) * 8, c = 2 * t + (e & 1);
     if (r < rows && c < nrhs) Y[(int64_t)(r0 + r) * ldy + c] = out[e];
+  }
   }
   // CTA barrier, then thread 0's release store: the rows written above are
   // visible to every CTA that acquires the counter
   __syncthreads();
-  if (tid == 0) st_release_s32(&flags[0], tk + 1);
+  if (tid == 0) st_release_s32(progress, tk + 1);
 }
 
 // G = -Lam * X^T (n x n), Lam and X n x k row-major, k <= 16: the rank-k
@@ -758,7 +864,7 @@ int pipe_attr() {
 
 template <typename TS>
 int launch_trsm_pipe(const TS* LU, int64_t lda, int n, double* Y, int64_t ldy, int nrhs, int mode, int* flags,
-                     unsigned* ticket, DevStatus* st, long long spin, cudaStream_t s) {
+                     DevStatus* st, long long spin, cudaStream_t s) {
   if (n <= 0 || nrhs <= 0) return LU_OK;
   // factor rows are staged in 16-byte chunks
   if (((lda * (int64_t)sizeof(TS)) & 15) || (reinterpret_cast<uintptr_t>(LU) & 15)) return LU_ERR_ALIGN;
@@ -770,13 +876,12 @@ int launch_trsm_pipe(const TS* LU, int64_t lda, int n, double* Y, int64_t ldy, i
   const int nblk = ceil_div(n, TB);
   for (int c0 = 0; c0 < nrhs; c0 += 16) {
     const int k = std::min(16, nrhs - c0);
-    LUB_CUDA(cudaMemsetAsync(flags, 0, sizeof(int), s));  // progress counter
-    LUB_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), s));
+    LUB_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * kPipeScratchInts, s));
     switch (mode) {
-      case 0: trsm_pipe_kernel<TS, 0><<<nblk, 256, smem, s>>>(LU, lda, n, Y + c0, ldy, k, flags, ticket, st, spin); break;
-      case 1: trsm_pipe_kernel<TS, 1><<<nblk, 256, smem, s>>>(LU, lda, n, Y + c0, ldy, k, flags, ticket, st, spin); break;
-      case 2: trsm_pipe_kernel<TS, 2><<<nblk, 256, smem, s>>>(LU, lda, n, Y + c0, ldy, k, flags, ticket, st, spin); break;
-      case 3: trsm_pipe_kernel<TS, 3><<<nblk, 256, smem, s>>>(LU, lda, n, Y + c0, ldy, k, flags, ticket, st, spin); break;
+      case 0: trsm_pipe_kernel<TS, 0><<<nblk * ceil_div(k, 8), 256, smem, s>>>(LU, lda, n, Y + c0, ldy, k, flags, st, spin); break;
+      case 1: trsm_pipe_kernel<TS, 1><<<nblk * ceil_div(k, 8), 256, smem, s>>>(LU, lda, n, Y + c0, ldy, k, flags, st, spin); break;
+      case 2: trsm_pipe_kernel<TS, 2><<<nblk * ceil_div(k, 8), 256, smem, s>>>(LU, lda, n, Y + c0, ldy, k, flags, st, spin); break;
+      case 3: trsm_pipe_kernel<TS, 3><<<nblk * ceil_div(k, 8), 256, smem, s>>>(LU, lda, n, Y + c0, ldy, k, flags, st, spin); break;
       default: return LU_ERR_ARG;
     }
     LUB_LAUNCH_CHECK();
@@ -857,7 +962,7 @@ int launch_trsm_wide(const float* L, int64_t ldl, float* B, int64_t ldb, int w, 
 }
 
 template <typename TS, typename T>
-int launch_trsv_mixed(const TS* LU, int64_t lda, int n, T* x, int upper, int* flags, unsigned* ticket, DevStatus* st,
+int launch_trsv_mixed(const TS* LU, int64_t lda, int n, T* x, int upper, int* flags, DevStatus* st,
                       long long spin, cudaStream_t s) {
   if (n <= 0) return LU_OK;
   const int nblk = ceil_div(n, TB);
@@ -871,34 +976,33 @@ int launch_trsv_mixed(const TS* LU, int64_t lda, int n, T* x, int upper, int* fl
           cudaFuncSetAttribute(trsv_kernel<TS, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return r;
   }));
-  // flags[0] is the progress counter; the ticket hands out block order
-  LUB_CUDA(cudaMemsetAsync(flags, 0, sizeof(int), s));
-  LUB_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), s));
+  // flags[0] is the progress counter, flags[1] the ticket that hands out block order
+  LUB_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * kTrsvScratchInts, s));
   if (upper)
-    trsv_kernel<TS, T, true><<<nblk, 256, smem, s>>>(LU, lda, n, x, flags, ticket, st, spin);
+    trsv_kernel<TS, T, true><<<nblk, 256, smem, s>>>(LU, lda, n, x, flags, st, spin);
   else
-    trsv_kernel<TS, T, false><<<nblk, 256, smem, s>>>(LU, lda, n, x, flags, ticket, st, spin);
+    trsv_kernel<TS, T, false><<<nblk, 256, smem, s>>>(LU, lda, n, x, flags, st, spin);
   LUB_LAUNCH_CHECK();
   return LU_OK;
 }
 
 template <typename T>
-int launch_trsv(const T* LU, int64_t lda, int n, T* x, int upper, int* flags, unsigned* ticket, DevStatus* st,
+int launch_trsv(const T* LU, int64_t lda, int n, T* x, int upper, int* flags, DevStatus* st,
                 long long spin, cudaStream_t s) {
-  return launch_trsv_mixed<T, T>(LU, lda, n, x, upper, flags, ticket, st, spin, s);
+  return launch_trsv_mixed<T, T>(LU, lda, n, x, upper, flags, st, spin, s);
 }
-template int launch_trsv_mixed<float, double>(const float*, int64_t, int, double*, int, int*, unsigned*, DevStatus*,
+template int launch_trsv_mixed<float, double>(const float*, int64_t, int, double*, int, int*, DevStatus*,
                                               long long, cudaStream_t);
 
-template int launch_trsm_pipe<double>(const double*, int64_t, int, double*, int64_t, int, int, int*, unsigned*,
+template int launch_trsm_pipe<double>(const double*, int64_t, int, double*, int64_t, int, int, int*,
                                       DevStatus*, long long, cudaStream_t);
-template int launch_trsm_pipe<float>(const float*, int64_t, int, double*, int64_t, int, int, int*, unsigned*,
+template int launch_trsm_pipe<float>(const float*, int64_t, int, double*, int64_t, int, int, int*,
                                      DevStatus*, long long, cudaStream_t);
 template int launch_trsm_llu_leaf<double>(const double*, int64_t, double*, int64_t, int, int, cudaStream_t);
 template int launch_trsm_llu_leaf<float>(const float*, int64_t, float*, int64_t, int, int, cudaStream_t);
-template int launch_trsv<double>(const double*, int64_t, int, double*, int, int*, unsigned*, DevStatus*, long long,
+template int launch_trsv<double>(const double*, int64_t, int, double*, int, int*, DevStatus*, long long,
                                  cudaStream_t);
-template int launch_trsv<float>(const float*, int64_t, int, float*, int, int*, unsigned*, DevStatus*, long long,
+template int launch_trsv<float>(const float*, int64_t, int, float*, int, int*, DevStatus*, long long,
                                 cudaStream_t);
 
 }  // namespace lub
