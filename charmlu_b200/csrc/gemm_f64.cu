@@ -7,10 +7,15 @@
 // kernel serves the GEMM halves of the recursive panel and TRSM.
 //
 // tcgen05 has no FP64 kind, so FP64 runs on mma.sync.m16n8k4.f64.
-// Tiling: CTA 128 x 128, K-tile 16, 4 stages; 8 warps as 2 (m) x 4 (n),
-// warp tile 64 x 32 = 4 x 4 DMMA tiles.  Shared-memory layout is what TMA's
-// 128-byte swizzle writes: A stage = 128 rows x 128 B; B stage = 8 column
-// slabs of 16 k-rows x 16 doubles.  Bank-conflict-free fragment loads come
+// Tiling: CTA 128 x 64, K-tile 16, 4 stages; 4 warps as 2 (m) x 2 (n),
+// warp tile 64 x 32 = 4 x 4 DMMA tiles; two CTAs per SM, so one loads and
+// stores its C tile while the other keeps the pipe busy.  What bounds it: the
+// DMMA pipe, but for those loads and stores: at K = 256 they are a tenth of a
+// tile's time.  16384 x 16384 x 256: one 128 x 128 CTA per SM 31.2 TFLOP/s, two
+// of 128 x 64 31.5, with their tiles half a tile apart 32.7 (K = 128: 28.2 ->
+// 30.2; K = 2048: 35.1).  Shared-memory layout is what TMA's 128-byte swizzle
+// writes: A stage = 128 rows x 128 B; B stage = 4 column slabs of 16 k-rows x
+// 16 doubles.  Bank-conflict-free fragment loads come
 // from two free choices of the MMA:
 //   * k order: in k-step s the lane with k-index t uses physical column
 //     2t + (s&1) + 8(s>>1), so a lane's A values for s = 0,1 (and 2,3) are
@@ -28,9 +33,9 @@
 namespace lub {
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 16, STAGES = 4, THREADS = 256;
+constexpr int BM = 128, BN = 64, BK = 16, STAGES = 4, THREADS = 128;
 constexpr int A_STAGE_BYTES = BM * BK * 8;          // 16 KB
-constexpr int B_STAGE_BYTES = BK * BN * 8;          // 16 KB
+constexpr int B_STAGE_BYTES = BK * BN * 8;          // 8 KB
 constexpr int STAGE_BYTES = A_STAGE_BYTES + B_STAGE_BYTES;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 128 /*barriers*/;
 
@@ -43,7 +48,7 @@ __device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, doubl
 
 __device__ __forceinline__ int mrow_perm(int g) { return (g >> 1) | ((g & 1) << 2); }
 
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __launch_bounds__(THREADS, 2)
 gemm_f64_sub_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                     GemmArgs args) {
   extern __shared__ unsigned char smem_raw[];
@@ -54,7 +59,7 @@ gemm_f64_sub_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int wm = warp >> 2, wn = warp & 3;
+  const int wm = warp >> 1, wn = warp & 1;
   int tm, tn;
   grouped_tile(blockIdx.x, (args.M + BM - 1) / BM, (args.N + BN - 1) / BN, 16, tm, tn);
   const int tile_m = tm * BM, tile_n = tn * BN;
@@ -62,6 +67,14 @@ gemm_f64_sub_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   const int KT = (K + BK - 1) / BK;
 
   if (tid == 0) {
+    // the first CTA in an SM's second slot starts about half a tile later:
+    // without that both CTAs of an SM load and store C at the same times
+    if (gridDim.x >= 8 * kNumSMsB200 && blockIdx.x < 2 * kNumSMsB200) {
+      unsigned w;
+      asm volatile("mov.u32 %0, %%warpid;" : "=r"(w));
+      if ((w / (THREADS / 32)) & 1)
+        for (int i = 0; i < KT; i++) __nanosleep(550);
+    }
     prefetch_tmap(&mapA);
     prefetch_tmap(&mapB);
     for (int s = 0; s < STAGES; s++) {
