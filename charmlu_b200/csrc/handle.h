@@ -75,6 +75,10 @@ struct lu_handle_s {
   // leaf tuning: recursion leaf width and CTA cap, without / with look-ahead
   int leaf_w64 = 32, leaf_w32 = 64, leaf_ctas = 148;
   int leaf_w64_la = 16, leaf_w32_la = 32, leaf_ctas_la = 48;
+  // FP64 look-ahead: the panel is hidden behind the update whatever its width,
+  // so its leaves take as few SMs from it as their rows allow (n = 32768: 48
+  // CTAs 825 ms, 24 816, 16 812)
+  int leaf_ctas_la64 = 16;
   // look-ahead is used while more than this many rows are left
   // (LU_B200_LA_MIN).  B200: FP64 n = 4999 23.1 ms with look-ahead to the end,
   // 19.5 without; n = 16384 141.8 / 137.4 with 6144 / 141.9 with 10240; mixed

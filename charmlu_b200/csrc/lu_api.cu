@@ -220,7 +220,7 @@ int factor_f64_schedule(lu_handle h, double* dA, int64_t lda, int32_t* ipiv, dou
   Ctx64 cp = c;
   cp.s = h->sP;
   cp.pl = h->plistP;
-  cp.leaf_ctas = h->leaf_ctas_la;
+  cp.leaf_ctas = h->leaf_ctas_la64;
   cp.alone = false;
   // under capture the panel stream's kernel nodes are marked for its priority
   std::vector<cudaGraphNode_t> mark;
@@ -343,7 +343,7 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
   h->leaf_ctas = h->num_sms;
   h->gemm_ctas = h->num_sms;
   if (const char* e = getenv("LU_B200_LEAF_CTAS")) h->leaf_ctas = std::max(1, atoi(e));
-  if (const char* e = getenv("LU_B200_LEAF_CTAS_LA")) h->leaf_ctas_la = std::max(1, atoi(e));
+  if (const char* e = getenv("LU_B200_LEAF_CTAS_LA")) h->leaf_ctas_la = h->leaf_ctas_la64 = std::max(1, atoi(e));
   if (const char* e = getenv("LU_B200_LEAF_W64")) h->leaf_w64 = std::min(32, std::max(2, atoi(e)));
   if (const char* e = getenv("LU_B200_LEAF_W64_LA")) h->leaf_w64_la = std::min(32, std::max(2, atoi(e)));
   if (const char* e = getenv("LU_B200_LEAF_W32")) h->leaf_w32 = std::min(64, std::max(4, atoi(e)));
@@ -653,7 +653,7 @@ Ctx64 block_ctx(lu_handle h, cudaStream_t s) {
   c.thr = h->cfg.sing_threshold;
   c.pl = h->plist;
   c.leaf_w = la ? h->leaf_w64_la : h->leaf_w64;
-  c.leaf_ctas = la ? h->leaf_ctas_la : h->leaf_ctas;
+  c.leaf_ctas = la ? h->leaf_ctas_la64 : h->leaf_ctas;
   c.alone = !la;
   return c;
 }
