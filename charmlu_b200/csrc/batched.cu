@@ -20,8 +20,8 @@
 // registers and rename rows instead of moving them (panel_regs); a panel of an
 // outer block is brought up to date as it is loaded; interchanges, U rows and
 // trailing update of an outer block go over the matrix together.
-// B200, 4096 systems of order 32 .. 1024 (log-uniform): FP64 64.5 -> 41.4 ms,
-// FP32 with refinement 71.9 -> 39.4 ms; one system of order 1024 on every SM:
+// B200, 4096 systems of order 32 .. 1024 (log-uniform): FP64 64.5 -> 39.7 ms,
+// FP32 with refinement 71.9 -> 39.6 ms; one system of order 1024 on every SM:
 // FP64 14.3 -> 9.4 ms (trailing update 4.6, panels 1.2 + 0.9 for loading and
 // storing them, U rows of the outer blocks 1.0, substitution 0.8).  Results are
 // bit for bit those of the right-looking form with plain fmas that it
@@ -153,7 +153,7 @@ __device__ __forceinline__ void dmma_k4(double (&c)[4], double a0, double a1, do
 // renames two rows, the CTA's candidate takes one barrier per column.  On
 // return lb holds the multipliers by original row, urow[j][i] = U(j, j + i),
 // sh.src[d] = the original row at position d.  Returns the 1-based first
-// column without a usable pivot (0: none).  rowbuf: [2][NWARP][W].
+// column without a usable pivot (0: none).  rowbuf: [2][NWARP][W] (FP32 only).
 template <typename T, int W, int RPT>
 __device__ __noinline__ int panel_regs(T* lb, int mp, int m, int kw, T* rowbuf, T* urow, T* zero, BShared<T>& sh) {
   constexpr int V = 16 / (int)sizeof(T);
@@ -174,33 +174,41 @@ __device__ __noinline__ int panel_regs(T* lb, int mp, int m, int kw, T* rowbuf, 
   for (int j = 0; j < steps; j++) {
     const int buf = j & 1;
     T* rows = rowbuf + buf * NWARP * W;
-    {
-      T bv = 0;
-      int bp = -1, bu = 0;
+    T bv = 0;
+    int bp = -1, bu = 0;
 #pragma unroll
-      for (int u = 0; u < RPT; u++) {
-        const T x = fabs(v[u][0]);
-        if (pos[u] >= 0 && (x > bv || (x == bv && bp >= 0 && pos[u] < bp))) {
-          bv = x;
-          bp = pos[u];
-          bu = u;
-        }
+    for (int u = 0; u < RPT; u++) {
+      const T x = fabs(v[u][0]);
+      if (pos[u] >= 0 && (x > bv || (x == bv && bp >= 0 && pos[u] < bp))) {
+        bv = x;
+        bp = pos[u];
+        bu = u;
       }
-      const int wl = warp_best(bv, bp >= 0, bp);
-      if (lane == max(wl, 0)) {
-        sh.key[buf][warp] = bv;
-        sh.pos[buf][warp] = wl < 0 ? -1 : bp;
+    }
+    const int wl = warp_best(bv, bp >= 0, bp);
+    // One lane stores 4 bytes a cycle.  FP64: sixteen candidates' rows would take
+    // longer than a second barrier, so only the best row is written, once it
+    // is known (4096 systems 41.5 -> 39.7 ms); FP32 rows are half as long and
+    // are written ahead (39.6 ms, 40.8 the other way)
+    constexpr bool kAheadRows = sizeof(T) == 4;
+    auto put_row = [&](T* dst) {
 #pragma unroll
-        for (int u = 0; u < RPT; u++)
-          if (RPT == 1 || bu == u) {
+      for (int u = 0; u < RPT; u++)
+        if (RPT == 1 || bu == u) {
 #pragma unroll
-            for (int i = 0; i < W; i += V) {
+          for (int i = 0; i < W; i += V) {
+            if (kAheadRows || i < W - j) {
               int4 q;
               memcpy(&q, &v[u][i], 16);
-              *reinterpret_cast<int4*>(&rows[warp * W + i]) = q;
+              *reinterpret_cast<int4*>(dst + i) = q;
             }
           }
-      }
+        }
+    };
+    if (lane == max(wl, 0)) {
+      sh.key[buf][warp] = bv;
+      sh.pos[buf][warp] = wl < 0 ? -1 : bp;
+      if (kAheadRows) put_row(rows + warp * W);
     }
     __syncthreads();
     const T ck = lane < NWARP ? sh.key[buf][lane] : T(0);
@@ -208,7 +216,11 @@ __device__ __noinline__ int panel_regs(T* lb, int mp, int m, int kw, T* rowbuf, 
     const int cw = warp_best(ck, cp >= 0, cp);
     const bool none = cw < 0;
     const int p = none ? j : sh.pos[buf][max(cw, 0)];
-    const T* pr = none ? zero : rows + max(cw, 0) * W;
+    if (!kAheadRows) {
+      if (warp == cw && lane == wl) put_row(urow + j * W);
+      __syncthreads();
+    }
+    const T* pr = none ? zero : (kAheadRows ? rows + max(cw, 0) * W : urow + j * W);
     if (none) {
       if (info == 0) info = j + 1;
 #pragma unroll
@@ -217,7 +229,7 @@ __device__ __noinline__ int panel_regs(T* lb, int mp, int m, int kw, T* rowbuf, 
 #pragma unroll
           for (int i = 0; i < W; i++) urow[j * W + i] = v[u][i];
         }
-    } else if (warp == (j & (NWARP - 1))) {
+    } else if (kAheadRows && warp == (j & (NWARP - 1))) {
       for (int k = lane; k < W; k += 32) urow[j * W + k] = pr[k];
     }
     const T piv = pr[0];
@@ -735,13 +747,13 @@ __device__ __forceinline__ void outer_update(T* A, int n, int K0, int nb, unsign
 // LU of an n x n system in shared memory (n <= the bucket's threshold):
 // a[c * mp + r], 16-column panels, everything right of a panel updated by one
 // fma per element and column in column order, as the unblocked elimination
-// does.  scr: rowbuf, urow and zero of panel_regs.
+// does.
 template <typename T>
 __device__ int factor_small(T* A, int n, unsigned char* smem, BShared<T>& sh) {
   constexpr int W = 16;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, mp = n | 1;
   T* a = reinterpret_cast<T*>(smem);
-  T* rowbuf = &sh.diag[0][0];  // 2 * NWARP * W + W * W + W <= 32 * 33 elements
+  T* rowbuf = &sh.diag[0][0];
   T* urow = rowbuf + 2 * NWARP * W;
   T* zero = urow + W * W;
   static_assert(2 * NWARP * W + W * W + W <= 32 * 33, "");
@@ -857,7 +869,7 @@ __device__ int factor_system(T* A, int n, unsigned char* smem, BShared<T>& sh) {
     const int W = kw <= 8 && sizeof(T) == 8 ? 8 : (kw <= 16 ? 16 : 32);
     T* lb = ut + ((Kp * up + 3) & ~3);  // [kw][mp]
     T* rowbuf = lb + ((kw * mp + 3) & ~3);
-    T* urow = rowbuf + 2 * NWARP * W;
+    T* urow = rowbuf + (sizeof(T) == 4 ? 2 * NWARP * W : 0);
     T* zero = urow + W * W;
     if (Kp == 0)
       for (int i = tid; i < n - K0; i += BT) sh.ob[i] = (unsigned short)i;
