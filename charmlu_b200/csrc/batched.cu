@@ -1195,20 +1195,50 @@ __global__ void __launch_bounds__(1024) batched_prep_kernel(int count, const int
     atomicAdd(&hist[v], 1);
   }
   __syncthreads();
+  // start position of every order, descending: an exclusive scan of the
+  // histogram from its end, two bins a thread; the offsets are a block scan
+  // too.  One thread's loops over both took 125 us of a call at 4096 systems
+  // (4096 systems of order 1: 0.306 -> 0.180 ms) and 35 us at 1000
+  static_assert(kBatchMaxN == 2048, "two bins per thread");
+  __shared__ long long w1[32], w2[32];
+  __shared__ int wb[32];
+  const int lane = tid & 31, warp = tid >> 5;
+  const int v0 = kBatchMaxN - 2 * tid;  // bins v0, v0 - 1
+  const int h0 = hist[v0], h1 = hist[v0 - 1];
+  int hs = h0 + h1;
+  // offsets of the systems: each thread a run of them
+  const int per = (count + 1023) / 1024, i0 = min(count, tid * per), i1 = min(count, i0 + per);
+  long long s1 = 0, s2 = 0;
+  for (int i = i0; i < i1; i++) {
+    const int v = n[i];
+    if (v >= 1 && v <= kBatchMaxN) { s2 += (long long)v * v; s1 += v; }
+  }
+  const int hown = hs;
+  const long long own1 = s1, own2 = s2;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, hs, o);
+    const long long b1 = __shfl_up_sync(0xffffffffu, s1, o), b2 = __shfl_up_sync(0xffffffffu, s2, o);
+    if (lane >= o) { hs += a; s1 += b1; s2 += b2; }
+  }
+  if (lane == 31) { wb[warp] = hs; w1[warp] = s1; w2[warp] = s2; }
+  __syncthreads();
+  int hb = 0;
+  long long t1 = 0, t2 = 0;
+  for (int w = 0; w < warp; w++) { hb += wb[w]; t1 += w1[w]; t2 += w2[w]; }
+  hist[v0] = hb + hs - hown;
+  hist[v0 - 1] = hb + hs - hown + h0;
+  long long p1 = t1 + s1 - own1, p2 = t2 + s2 - own2;
+  for (int i = i0; i < i1; i++) {
+    const int v = n[i];
+    offA32[i] = p2;
+    offV[i] = p1;
+    if (v >= 1 && v <= kBatchMaxN) { p2 += (long long)v * v; p1 += v; }
+  }
   if (tid == 0) {
-    int acc = 0;  // descending start positions
-    for (int v = kBatchMaxN; v >= 1; v--) {
-      const int c = hist[v];
-      hist[v] = acc;
-      acc += c;
-    }
-    long long s2 = 0, s1 = 0;
-    for (int i = 0; i < count; i++) {
-      const int v = n[i];
-      offA32[i] = s2;
-      offV[i] = s1;
-      if (v >= 1 && v <= kBatchMaxN) { s2 += (long long)v * v; s1 += v; }
-    }
+    s1 = 0;
+    s2 = 0;
+    for (int w = 0; w < 32; w++) { s1 += w1[w]; s2 += w2[w]; }
     hdr->queue = 0;
     for (int q = 0; q < kRefineHistBins; q++) hdr->refine_hist[q] = 0;
     hdr->s1 = s1;
