@@ -18,8 +18,8 @@ namespace {
 constexpr int BM = 128, BN = 128, BK = 16, THREADS = 256;
 
 __global__ void __launch_bounds__(THREADS, 2)
-gemm_f32_sub_kernel(const float* __restrict__ A, int64_t lda, const float* __restrict__ B, int64_t ldb,
-                    float* __restrict__ C, int64_t ldc, int M, int N, int K) {
+gemm_f32_sub_kernel(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc, int M, int N,
+                    int K) {
   __shared__ __align__(16) float As[2][BK][BM + 4];
   __shared__ __align__(16) float Bs[2][BK][BN + 4];
   const int tid = threadIdx.x;
@@ -31,6 +31,7 @@ gemm_f32_sub_kernel(const float* __restrict__ A, int64_t lda, const float* __res
   // B tile 16 x 128 -> each thread 8 elements (k rows bk, bk+8; cols bn..bn+3)
   const int bk = tid >> 5, bn = (tid & 31) * 4;
 
+  after_previous_kernel();
   float ra[2][4], rb[2][4];
   auto load = [&](int k0) {
 #pragma unroll
@@ -39,13 +40,13 @@ gemm_f32_sub_kernel(const float* __restrict__ A, int64_t lda, const float* __res
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         const int k = k0 + ak + e;
-        ra[h][e] = (r < M && k < K) ? __ldg(&A[(int64_t)r * lda + k]) : 0.f;
+        ra[h][e] = (r < M && k < K) ? A[(int64_t)r * lda + k] : 0.f;
       }
       const int kb = k0 + bk + h * 8;
 #pragma unroll
       for (int e = 0; e < 4; e++) {
         const int c = tn + bn + e;
-        rb[h][e] = (kb < K && c < N) ? __ldg(&B[(int64_t)kb * ldb + c]) : 0.f;
+        rb[h][e] = (kb < K && c < N) ? B[(int64_t)kb * ldb + c] : 0.f;
       }
     }
   };
@@ -116,8 +117,8 @@ constexpr int NBM = 64, NKMAX = 64, NTHREADS = 256;
 
 template <int BN, bool CHAIN = false>
 __global__ void __launch_bounds__(NTHREADS)
-gemm_f32_narrow_kernel(const float* __restrict__ A, int64_t lda, const float* __restrict__ B, int64_t ldb,
-                       float* __restrict__ C, int64_t ldc, int M, int N, int K) {
+gemm_f32_narrow_kernel(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc, int M, int N,
+                       int K) {
   constexpr int QN = BN / 4;           // column quads
   constexpr int RG = NTHREADS / QN;    // row groups
   constexpr int RPT = NBM / RG;        // rows per thread
@@ -126,13 +127,14 @@ gemm_f32_narrow_kernel(const float* __restrict__ A, int64_t lda, const float* __
   const int tid = threadIdx.x;
   const int tx = tid % QN, ty = tid / QN;
   const int row0 = blockIdx.x * NBM;
+  after_previous_kernel();
   for (int idx = tid; idx < K * BN; idx += NTHREADS) {
     const int k = idx / BN, c = idx - k * BN;
-    Bs[k][c] = c < N ? __ldg(&B[(int64_t)k * ldb + c]) : 0.f;
+    Bs[k][c] = c < N ? B[(int64_t)k * ldb + c] : 0.f;
   }
   for (int idx = tid; idx < NBM * K; idx += NTHREADS) {
     const int r = idx / K, k = idx - r * K;
-    As[r][k] = row0 + r < M ? __ldg(&A[(int64_t)(row0 + r) * lda + k]) : 0.f;
+    As[r][k] = row0 + r < M ? A[(int64_t)(row0 + r) * lda + k] : 0.f;
   }
   __syncthreads();
   float acc[RPT][4];
@@ -175,17 +177,11 @@ static int gemm_f32_dispatch(const float* A, int64_t lda, const float* B, int64_
                              int N, int K, bool allow_narrow, cudaStream_t s) {
   if (M <= 0 || N <= 0 || K <= 0) return LU_OK;
   if (allow_narrow && K <= NKMAX && N <= 64) {
-    if (N <= 32)
-      gemm_f32_narrow_kernel<32><<<ceil_div(M, NBM), NTHREADS, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K);
-    else
-      gemm_f32_narrow_kernel<64><<<ceil_div(M, NBM), NTHREADS, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K);
-    LUB_LAUNCH_CHECK();
-    return LU_OK;
+    return launch_dependent(N <= 32 ? gemm_f32_narrow_kernel<32> : gemm_f32_narrow_kernel<64>,
+                            dim3(ceil_div(M, NBM)), dim3(NTHREADS), 0, s, A, lda, B, ldb, C, ldc, M, N, K);
   }
   dim3 grid(ceil_div(N, BN), ceil_div(M, BM));
-  gemm_f32_sub_kernel<<<grid, THREADS, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K);
-  LUB_LAUNCH_CHECK();
-  return LU_OK;
+  return launch_dependent(gemm_f32_sub_kernel, grid, dim3(THREADS), 0, s, A, lda, B, ldb, C, ldc, M, N, K);
 }
 
 int launch_gemm_f32_sub(const float* A, int64_t lda, const float* B, int64_t ldb, float* C, int64_t ldc, int M,
@@ -197,9 +193,8 @@ int launch_gemm_f32_chain(const float* A, int64_t lda, const float* B, int64_t l
                           int N, int K, cudaStream_t s) {
   if (M <= 0 || N <= 0 || K <= 0) return LU_OK;
   if (N > 32 || K > NKMAX) return LU_ERR_ARG;
-  gemm_f32_narrow_kernel<32, true><<<ceil_div(M, NBM), NTHREADS, 0, s>>>(A, lda, B, ldb, C, ldc, M, N, K);
-  LUB_LAUNCH_CHECK();
-  return LU_OK;
+  return launch_dependent(gemm_f32_narrow_kernel<32, true>, dim3(ceil_div(M, NBM)), dim3(NTHREADS), 0, s, A, lda, B,
+                          ldb, C, ldc, M, N, K);
 }
 
 }  // namespace lub

@@ -84,6 +84,7 @@ gemm_f64_sub_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
     fence_mbar_init();
   }
   __syncthreads();
+  after_previous_kernel();
 
   auto issue = [&](int kt, int s) {
     unsigned char* sa = smem + s * STAGE_BYTES;
@@ -235,9 +236,7 @@ int launch_gemm_f64_sub(const CUtensorMap& mapA, const CUtensorMap& mapB, const 
     return LU_ERR_ALIGN;
   const int64_t tiles = (int64_t)ceil_div(a.N, BN) * ceil_div(a.M, BM);
   if (tiles > INT32_MAX) return LU_ERR_UNSUPPORTED;
-  gemm_f64_sub_kernel<<<(unsigned)tiles, THREADS, SMEM_BYTES, stream>>>(mapA, mapB, a);
-  LUB_LAUNCH_CHECK();
-  return LU_OK;
+  return launch_dependent(gemm_f64_sub_kernel, dim3((unsigned)tiles), dim3(THREADS), SMEM_BYTES, stream, mapA, mapB, a);
 }
 
 }  // namespace lub

@@ -179,6 +179,7 @@ __global__ void __launch_bounds__(NT, 1) getf2_leaf_kernel(T* P, T* prow0, LeafA
   const int G = XP == kSingle ? 1 : gridDim.x, cta = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r_lo = cta * a.R, nr = min(a.M, r_lo + a.R) - r_lo, ncols = a.ncols;
   const bool vec = ncols == W && a.lda % V == 0 && (reinterpret_cast<uintptr_t>(P) & 15) == 0;
+  if constexpr (XP != kGrid) after_previous_kernel();
 
   // ---- rows into registers
   T v[RPT][W];
@@ -542,18 +543,20 @@ int launch_leaf(T* P, T* prow0, const LeafArgs& a, int G, cudaStream_t s) {
     cfg.blockDim = dim3(NT);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = G;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = may_overlap_launch(s) ? 2 : 1;
     LUB_CUDA(cudaLaunchKernelExC(&cfg, fn, ptrs));
   } else if (XP == kGrid) {
     LUB_CUDA(cudaLaunchCooperativeKernel(fn, dim3(G), dim3(NT), ptrs, smem, s));
   } else {
-    LUB_CUDA(cudaLaunchKernel(fn, dim3(1), dim3(NT), ptrs, smem, s));
+    return launch_dependent(getf2_leaf_kernel<T, W, RPT, XP>, dim3(1), dim3(NT), smem, s, P, prow0, a);
   }
   __atomic_add_fetch(&g_kernel_launches, 1, __ATOMIC_RELAXED);
   return LU_OK;

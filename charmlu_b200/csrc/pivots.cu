@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(1024) pivot_compose_kernel(const int32_t* ipiv
   __shared__ int p[kMaxBatch], nxt[kMaxBatch], lb[kMaxBatch];
   __shared__ int dst[2 * kMaxBatch], src[2 * kMaxBatch];
   __shared__ int s_m;
+  after_previous_kernel();
   if (rows > 0) {
     int bad = k0 + cnt > rows;
     for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
@@ -125,6 +126,7 @@ __global__ void __launch_bounds__(kApplyThreads) pivot_apply_kernel(T* A, int64_
   constexpr int CS = 8 * EPC;               // elements per strip
   __shared__ double vb[2 * kMaxBatch];
   __shared__ int32_t pb[2 * kMaxBatch];
+  after_previous_kernel();
   const int m = *pl.m;
   const int tid = threadIdx.x;
   const int c0 = c_begin + blockIdx.x * CS;
@@ -243,9 +245,7 @@ int launch_pivot_compose(const int32_t* ipiv, int k0, int cnt, const PivotList& 
                          DevStatus* st) {
   if (cnt <= 0) return LU_OK;
   if (cnt > kMaxBatch) return LU_ERR_ARG;
-  pivot_compose_kernel<<<1, 1024, 0, s>>>(ipiv, k0, cnt, pl, rows, st);
-  LUB_LAUNCH_CHECK();
-  return LU_OK;
+  return launch_dependent(pivot_compose_kernel, dim3(1), dim3(1024), 0, s, ipiv, k0, cnt, pl, rows, st);
 }
 
 template <typename T>
@@ -257,10 +257,8 @@ int launch_pivot_apply(T* A, int64_t lda, int c_begin, int c_end, int skip_begin
   const int vec_ok = ((lda * (int64_t)sizeof(T)) % 16 == 0) && (reinterpret_cast<uintptr_t>(A) % 16 == 0) &&
                      (c_begin % (16 / (int)sizeof(T)) == 0);
   const int strips = std::max(1, ceil_div(std::max(c_end - c_begin, 0), CS));
-  pivot_apply_kernel<T><<<strips, kApplyThreads, 0, s>>>(A, lda, c_begin, c_end, skip_begin, skip_end, pl, rhs,
-                                                          perm, vec_ok);
-  LUB_LAUNCH_CHECK();
-  return LU_OK;
+  return launch_dependent(pivot_apply_kernel<T>, dim3(strips), dim3(kApplyThreads), 0, s, A, lda, c_begin, c_end,
+                          skip_begin, skip_end, pl, rhs, perm, vec_ok);
 }
 
 int ipiv_to_perm_work_ints(int n) { return ceil_div(std::max(n, 1), kPermBatch) * kPermListInts; }

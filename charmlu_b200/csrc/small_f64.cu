@@ -75,9 +75,8 @@ constexpr int GLP = GK + 8, GBP = GN + 2;
 constexpr int kSmallStage = GM * GLP + GK * GBP;  // doubles
 constexpr size_t kSmallSmem = 2 * kSmallStage * sizeof(double);
 
-__global__ void __launch_bounds__(GT) gemm_f64_small_kernel(const double* __restrict__ A, int64_t lda,
-                                                            const double* __restrict__ B, int64_t ldb, double* C,
-                                                            int64_t ldc, int M, int N, int K) {
+__global__ void __launch_bounds__(GT) gemm_f64_small_kernel(const double* A, int64_t lda, const double* B,
+                                                            int64_t ldb, double* C, int64_t ldc, int M, int N, int K) {
   extern __shared__ __align__(16) double smem_d[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int r0 = blockIdx.x * GM, c0 = blockIdx.y * GN;
@@ -101,6 +100,7 @@ __global__ void __launch_bounds__(GT) gemm_f64_small_kernel(const double* __rest
     }
     cp_commit();
   };
+  after_previous_kernel();
   stage(0);
   double acc[2][2][4];
   double* Cp[2][2];
@@ -161,7 +161,7 @@ constexpr size_t strip_smem(int w) {
 }
 
 template <int CB>
-__global__ void __launch_bounds__(ST) trsm_strip_kernel(const double* __restrict__ L, int64_t ldl, double* B,
+__global__ void __launch_bounds__(ST) trsm_strip_kernel(const double* L, int64_t ldl, double* B,
                                                         int64_t ldb, int w, int ncols,
                                                         const __grid_constant__ StripBlocks blk) {
   constexpr int XP = CB + 2;
@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(ST) trsm_strip_kernel(const double* __restrict
   double* X = smem_d;                     // [rows][XP]
   double* Lb[2] = {X + (size_t)rows * XP, X + (size_t)rows * XP + (size_t)rows * SLP};
   const int c0 = blockIdx.x * CB, nc = min(CB, ncols - c0);
+  after_previous_kernel();
   for (int idx = tid; idx < rows * (CB / 2); idx += ST) {
     const int r = idx / (CB / 2), c = (idx % (CB / 2)) * 2;
     const int live = r < w ? max(0, min(2, nc - c)) : 0;
@@ -282,9 +283,8 @@ int launch_strip(const double* L, int64_t ldl, double* B, int64_t ldb, int w, in
     return cuda_status(cudaFuncSetAttribute(trsm_strip_kernel<CB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)strip_smem<CB>(kStripW)));
   }));
-  trsm_strip_kernel<CB><<<ceil_div(ncols, CB), ST, strip_smem<CB>(w), s>>>(L, ldl, B, ldb, w, ncols, blk);
-  LUB_LAUNCH_CHECK();
-  return LU_OK;
+  return launch_dependent(trsm_strip_kernel<CB>, dim3(ceil_div(ncols, CB)), dim3(ST), strip_smem<CB>(w), s, L, ldl, B,
+                          ldb, w, ncols, blk);
 }
 
 }  // namespace
@@ -299,9 +299,7 @@ int launch_gemm_f64_small(const double* A, int64_t lda, const double* B, int64_t
   }));
   dim3 grid(ceil_div(M, GM), ceil_div(N, GN));
   if (grid.y > 65535) return LU_ERR_UNSUPPORTED;
-  gemm_f64_small_kernel<<<grid, GT, kSmallSmem, s>>>(A, lda, B, ldb, C, ldc, M, N, K);
-  LUB_LAUNCH_CHECK();
-  return LU_OK;
+  return launch_dependent(gemm_f64_small_kernel, grid, dim3(GT), kSmallSmem, s, A, lda, B, ldb, C, ldc, M, N, K);
 }
 
 int launch_trsm_f64_strip(const double* L, int64_t ldl, double* B, int64_t ldb, int w, int ncols, cudaStream_t s) {

@@ -28,6 +28,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) trsm_llu_leaf_kernel(const T* L, int64_t ldl, T* B, int64_t ldb, int m,
                                                             int ncols) {
   __shared__ T sL[32][33];
+  after_previous_kernel();
   for (int idx = threadIdx.x; idx < 32 * 32; idx += blockDim.x) {
     const int i = idx >> 5, p = idx & 31;
     sL[i][p] = (i < m && p < i) ? L[(int64_t)i * ldl + p] : T(0);
@@ -61,9 +62,8 @@ constexpr int kTrsmNT = 256;
 // CB columns of B per CTA (4 .. 32): narrow slices spread a small solve over
 // more SMs; each column's arithmetic is the same for every CB.
 template <int CB>
-__global__ void __launch_bounds__(kTrsmNT) trsm_llu_block_kernel(const float* __restrict__ L, int64_t ldl,
-                                                                 float* __restrict__ B, int64_t ldb, int w,
-                                                                 int ncols) {
+__global__ void __launch_bounds__(kTrsmNT) trsm_llu_block_kernel(const float* L, int64_t ldl, float* B,
+                                                                 int64_t ldb, int w, int ncols) {
   constexpr int TXN = CB / 4;          // groups of 4 columns
   constexpr int RS = kTrsmNT / TXN;    // rows updated in parallel
   __shared__ float sB[kTrsmBlockMaxW][CB + 1];
@@ -71,6 +71,7 @@ __global__ void __launch_bounds__(kTrsmNT) trsm_llu_block_kernel(const float* __
   const int tid = threadIdx.x;
   const int c0 = blockIdx.x * CB;
   const int nc = min(CB, ncols - c0);
+  after_previous_kernel();
   for (int idx = tid; idx < w * CB; idx += kTrsmNT) {
     const int r = idx / CB, c = idx - r * CB;
     sB[r][c] = c < nc ? B[(int64_t)r * ldb + c0 + c] : 0.f;
@@ -149,10 +150,10 @@ constexpr size_t kWideSmem =
 
 // dinv[b] (32 x 32, row-major) = inverse of the unit-lower diagonal block b
 // of L (w x w), rows / columns past w treated as identity
-__global__ void __launch_bounds__(32) tri_inv32_kernel(const float* __restrict__ L, int64_t ldl, int w,
-                                                       float* __restrict__ dinv) {
+__global__ void __launch_bounds__(32) tri_inv32_kernel(const float* L, int64_t ldl, int w, float* dinv) {
   __shared__ float sL[32][33];
   const int b = blockIdx.x, j = threadIdx.x, k0 = 32 * b, kb = min(32, w - k0);
+  after_previous_kernel();
 #pragma unroll 4
   for (int i = 0; i < 32; i++) sL[i][j] = (i < kb && j < i) ? L[(int64_t)(k0 + i) * ldl + k0 + j] : 0.f;
   __syncthreads();
@@ -236,9 +237,8 @@ __device__ __forceinline__ void wide_update8(float* sB, const float* Ls, int r0,
 
 // VEC: L, B, ldl and ldb allow 16-byte copies (else element loads)
 template <bool VEC>
-__global__ void __launch_bounds__(kWideNT, 1) trsm_wide_kernel(const float* __restrict__ L, int64_t ldl,
-                                                              const float* __restrict__ dinv, float* __restrict__ B,
-                                                              int64_t ldb, int w, int ncols) {
+__global__ void __launch_bounds__(kWideNT, 1) trsm_wide_kernel(const float* L, int64_t ldl, const float* dinv,
+                                                              float* B, int64_t ldb, int w, int ncols) {
   extern __shared__ __align__(16) float wide_smem[];
   float* sB = wide_smem;                                  // [32 nkb][kWideBP]
   float* sL = wide_smem + (size_t)kWideMaxW * kWideBP;    // [2][w - 32][kWideLP]
@@ -246,6 +246,7 @@ __global__ void __launch_bounds__(kWideNT, 1) trsm_wide_kernel(const float* __re
   const int tid = threadIdx.x;
   const int c0 = blockIdx.x * kWideCB, nc = min(kWideCB, ncols - c0);
   const int nkb = (w + 31) / 32, wp = nkb * 32;
+  after_previous_kernel();
   if (VEC && nc == kWideCB) {
     for (int idx = tid; idx < wp * 8; idx += kWideNT) {
       const int r = idx >> 3, q = idx & 7;
@@ -913,25 +914,19 @@ template <typename T>
 int launch_trsm_llu_leaf(const T* L, int64_t ldl, T* B, int64_t ldb, int m, int ncols, cudaStream_t s) {
   if (m <= 1 || ncols <= 0) return LU_OK;
   if (m > 32) return LU_ERR_ARG;
-  trsm_llu_leaf_kernel<T><<<ceil_div(ncols, 128), 128, 0, s>>>(L, ldl, B, ldb, m, ncols);
-  LUB_LAUNCH_CHECK();
-  return LU_OK;
+  return launch_dependent(trsm_llu_leaf_kernel<T>, dim3(ceil_div(ncols, 128)), dim3(128), 0, s, L, ldl, B, ldb, m,
+                          ncols);
 }
 
 int launch_trsm_llu_block(const float* L, int64_t ldl, float* B, int64_t ldb, int w, int ncols, cudaStream_t s) {
   if (w <= 1 || ncols <= 0) return LU_OK;
   if (w > kTrsmBlockMaxW) return LU_ERR_ARG;
   // slices narrow enough for at least ~32 CTAs
-  if (ncols >= 1024)
-    trsm_llu_block_kernel<32><<<ceil_div(ncols, 32), kTrsmNT, 0, s>>>(L, ldl, B, ldb, w, ncols);
-  else if (ncols >= 512)
-    trsm_llu_block_kernel<16><<<ceil_div(ncols, 16), kTrsmNT, 0, s>>>(L, ldl, B, ldb, w, ncols);
-  else if (ncols >= 256)
-    trsm_llu_block_kernel<8><<<ceil_div(ncols, 8), kTrsmNT, 0, s>>>(L, ldl, B, ldb, w, ncols);
-  else
-    trsm_llu_block_kernel<4><<<ceil_div(ncols, 4), kTrsmNT, 0, s>>>(L, ldl, B, ldb, w, ncols);
-  LUB_LAUNCH_CHECK();
-  return LU_OK;
+  const int cb = ncols >= 1024 ? 32 : ncols >= 512 ? 16 : ncols >= 256 ? 8 : 4;
+  const auto fn = cb == 32 ? trsm_llu_block_kernel<32>
+                  : cb == 16 ? trsm_llu_block_kernel<16>
+                  : cb == 8 ? trsm_llu_block_kernel<8> : trsm_llu_block_kernel<4>;
+  return launch_dependent(fn, dim3(ceil_div(ncols, cb)), dim3(kTrsmNT), 0, s, L, ldl, B, ldb, w, ncols);
 }
 
 // dinv: device scratch of 16 x 1024 floats (the diagonal-block inverses)
@@ -948,17 +943,12 @@ int launch_trsm_wide(const float* L, int64_t ldl, float* B, int64_t ldb, int w, 
     return LU_OK;
   }));
   const int nkb = ceil_div(w, 32);
-  tri_inv32_kernel<<<nkb, 32, 0, s>>>(L, ldl, w, dinv);
-  LUB_LAUNCH_CHECK();
+  LUB_TRY(launch_dependent(tri_inv32_kernel, dim3(nkb), dim3(32), 0, s, L, ldl, w, dinv));
   const bool vec = ((reinterpret_cast<uintptr_t>(L) | reinterpret_cast<uintptr_t>(B)) & 15) == 0 &&
                    (ldl & 3) == 0 && (ldb & 3) == 0;
   const unsigned grid = (unsigned)ceil_div(ncols, kWideCB);
-  if (vec)
-    trsm_wide_kernel<true><<<grid, kWideNT, kWideSmem, s>>>(L, ldl, dinv, B, ldb, w, ncols);
-  else
-    trsm_wide_kernel<false><<<grid, kWideNT, kWideSmem, s>>>(L, ldl, dinv, B, ldb, w, ncols);
-  LUB_LAUNCH_CHECK();
-  return LU_OK;
+  return launch_dependent(vec ? trsm_wide_kernel<true> : trsm_wide_kernel<false>, dim3(grid), dim3(kWideNT), kWideSmem, s,
+                          L, ldl, dinv, B, ldb, w, ncols);
 }
 
 template <typename TS, typename T>
