@@ -199,12 +199,7 @@ __global__ void __launch_bounds__(ST) trsm_strip_kernel(const double* L, int64_t
       double* xc = X + l0 * XP + tid;
 #pragma unroll
       for (int i = 0; i < 32; i++) x[i] = i < kb ? xc[i * XP] : 0.0;
-      // the staged columns past kb are zero, and so are the rows read past w
-#pragma unroll
-      for (int p = 0; p < 31; p++)
-#pragma unroll
-        for (int i = p + 1; i < 32; i++)
-          if (i < kb) x[i] = fma(-ls[i * SLP + p], x[p], x[i]);
+      solve_unit_lower32(x, ls, SLP, kb);
 #pragma unroll
       for (int i = 1; i < 32; i++)
         if (i < kb) xc[i * XP] = x[i];

@@ -27,23 +27,20 @@ namespace {
 template <typename T>
 __global__ void __launch_bounds__(128) trsm_llu_leaf_kernel(const T* L, int64_t ldl, T* B, int64_t ldb, int m,
                                                             int ncols) {
-  __shared__ T sL[32][33];
+  __shared__ __align__(16) T sL[32][36];
   after_previous_kernel();
-  for (int idx = threadIdx.x; idx < 32 * 32; idx += blockDim.x) {
-    const int i = idx >> 5, p = idx & 31;
+  const int col = blockIdx.x * blockDim.x + threadIdx.x;
+  T x[32];
+#pragma unroll
+  for (int i = 0; i < 32; i++) x[i] = i < m && col < ncols ? B[(int64_t)i * ldb + col] : T(0);
+#pragma unroll
+  for (int u = 0; u < 8; u++) {
+    const int idx = threadIdx.x + u * 128, i = idx >> 5, p = idx & 31;
     sL[i][p] = (i < m && p < i) ? L[(int64_t)i * ldl + p] : T(0);
   }
   __syncthreads();
-  const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= ncols) return;
-  T x[32];
-#pragma unroll
-  for (int i = 0; i < 32; i++) x[i] = i < m ? B[(int64_t)i * ldb + col] : T(0);
-#pragma unroll
-  for (int i = 1; i < 32; i++) {
-#pragma unroll
-    for (int p = 0; p < i; p++) x[i] = fma(-sL[i][p], x[p], x[i]);
-  }
+  solve_unit_lower32(x, &sL[0][0], 36, 32);
 #pragma unroll
   for (int i = 0; i < 32; i++)
     if (i < m) B[(int64_t)i * ldb + col] = x[i];
@@ -67,8 +64,9 @@ __global__ void __launch_bounds__(kTrsmNT) trsm_llu_block_kernel(const float* L,
   constexpr int TXN = CB / 4;          // groups of 4 columns
   constexpr int RS = kTrsmNT / TXN;    // rows updated in parallel
   __shared__ float sB[kTrsmBlockMaxW][CB + 1];
-  __shared__ float sL[32][33];
+  __shared__ __align__(16) float sL[32][36];
   const int tid = threadIdx.x;
+  const bool vec = (ldl & 3) == 0 && (reinterpret_cast<uintptr_t>(L) & 15) == 0;
   const int c0 = blockIdx.x * CB;
   const int nc = min(CB, ncols - c0);
   after_previous_kernel();
@@ -88,11 +86,7 @@ __global__ void __launch_bounds__(kTrsmNT) trsm_llu_block_kernel(const float* L,
       float x[32];
 #pragma unroll
       for (int i = 0; i < 32; i++) x[i] = i < kb ? sB[k0 + i][tid] : 0.f;
-#pragma unroll
-      for (int i = 1; i < 32; i++) {
-#pragma unroll
-        for (int p = 0; p < i; p++) x[i] = fmaf(-sL[i][p], x[p], x[i]);
-      }
+      solve_unit_lower32(x, &sL[0][0], 36, 32);
 #pragma unroll
       for (int i = 0; i < 32; i++)
         if (i < kb) sB[k0 + i][tid] = x[i];
@@ -103,8 +97,19 @@ __global__ void __launch_bounds__(kTrsmNT) trsm_llu_block_kernel(const float* L,
     for (int r = k0 + kb + ty; r < w; r += RS) {
       const float* lr = L + (int64_t)r * ldl + k0;
       float a0 = sB[r][4 * tx], a1 = sB[r][4 * tx + 1], a2 = sB[r][4 * tx + 2], a3 = sB[r][4 * tx + 3];
-      for (int p = 0; p < kb; p++) {
-        const float l = __ldg(&lr[p]);
+      float ll[32];  // rows below a block: its 32 columns are all there
+#pragma unroll
+      for (int p = 0; p < 32; p += 4) {
+        if (vec) {
+          const float4 q = *reinterpret_cast<const float4*>(lr + p);
+          ll[p] = q.x; ll[p + 1] = q.y; ll[p + 2] = q.z; ll[p + 3] = q.w;
+        } else {
+          ll[p] = lr[p]; ll[p + 1] = lr[p + 1]; ll[p + 2] = lr[p + 2]; ll[p + 3] = lr[p + 3];
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < 32; p++) {
+        const float l = ll[p];
         a0 = fmaf(-l, sB[k0 + p][4 * tx], a0);
         a1 = fmaf(-l, sB[k0 + p][4 * tx + 1], a1);
         a2 = fmaf(-l, sB[k0 + p][4 * tx + 2], a2);
