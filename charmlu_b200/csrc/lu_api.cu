@@ -674,7 +674,7 @@ int lu_panel_factor(lu_handle h, double* dP, int64_t ldp, int64_t m, int32_t w, 
   c.n = (int)m;
   c.base = (int)base;
   LUB_TRY(c.A.init(dP, m, w, ldp));
-  // one barrier counter per leaf, from a pool cleared for this panel
+  // one tag per leaf, distinct within this panel; packets and counters start cleared
   LUB_CUDA(cudaMemsetAsync(h->leaf_pkt, 0, h->clear_bytes(), s));
   h->next_counter = 0;
   return panel64(c, 0, w, 0, w);

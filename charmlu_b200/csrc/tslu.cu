@@ -1,7 +1,7 @@
 // Panel leaf with tournament pivoting (TSLU) for the FP32 panels of the
 // mixed-precision path.
 //
-// The partial-pivoting leaf (panel.cu) needs one grid-wide argmax per
+// The partial-pivoting leaf (panel.cuh) needs one grid-wide argmax per
 // column: a grid barrier and L2 round trips that cost ~5 us per column
 // whatever the panel height, which makes the panel chain the critical path
 // of the mixed factorisation.  Tournament pivoting (the TSLU panel of
