@@ -28,11 +28,14 @@ __global__ void __launch_bounds__(256) residual_f64_kernel(const double* A, int6
     const double* ar = A + (int64_t)lrow * lda;
     double s0 = 0.0, s1 = 0.0;
     const bool vec = ((lda & 1) == 0) && ((reinterpret_cast<uintptr_t>(A) & 15) == 0);
+    // x may stand at an odd offset (the Krylov basis of an odd order has its
+    // vectors n apart): then 8 bytes at a time, in the same order
+    const bool xvec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
     if (vec) {
       const int n2 = n & ~1;
       for (int j = lane * 2; j < n2; j += 64) {
         const double2 a = __ldcs(reinterpret_cast<const double2*>(ar + j));
-        const double2 xv = *reinterpret_cast<const double2*>(x + j);
+        const double2 xv = xvec ? *reinterpret_cast<const double2*>(x + j) : make_double2(x[j], x[j + 1]);
         s0 = fma(a.x, xv.x, s0);
         s1 = fma(a.y, xv.y, s1);
         rs += fabs(a.x) + fabs(a.y);

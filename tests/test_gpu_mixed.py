@@ -225,6 +225,28 @@ def test_gmres_ir_mode(cuda_dev):
     assert s.residual(A, x, rhs)["r_hpl"] < 16
 
 
+@pytest.mark.parametrize("n", [257, 1001])
+def test_gmres_odd_order(cuda_dev, n):
+    """Every other vector of the Krylov basis starts 8 bytes off a 16-byte
+    boundary, while the matrix is read 16 bytes at a time."""
+    import charmlu_b200 as lu
+    rng = np.random.default_rng(n)
+    A_np = rng.uniform(-0.5, 0.5, (n, n)) + np.eye(n) * np.sqrt(n)
+    b_np = rng.uniform(-0.5, 0.5, n)
+    A = torch.zeros(n, n + 1, dtype=torch.float64, device="cuda")[:, :n]
+    A.copy_(torch.from_numpy(A_np))
+    b = torch.from_numpy(b_np).cuda()
+    s = lu.LUSolver(lu.LUConfig(n, 64, precision=lu.LU_PREC_FP16X3, ir_mode=lu.LU_IR_GMRES))
+    x, info = s.refine_solve(A, b)
+    assert info["status"] == 0 and info["used_gmres"] == 1, info
+    ref = np.linalg.solve(A_np, b_np)
+    assert np.abs(x.cpu().numpy() - ref).max() <= 1e-10 * np.abs(ref).max()
+    # the residual takes a solution at such an address too
+    buf = torch.zeros(n + 1, dtype=torch.float64, device="cuda")
+    buf[1:].copy_(x)
+    assert s.residual(A, buf[1:], b)["r_hpl"] == s.residual(A, x, b)["r_hpl"]
+
+
 def test_singular_matrix_reports_info_mixed(cuda_dev):
     import charmlu_b200 as lu
     n, b = 256, 64
