@@ -227,6 +227,15 @@ struct lu_handle_s {
     *p = static_cast<T*>(q);
     return LU_OK;
   }
+  // Zeros in a new block before any stream may read it: a memset on the default
+  // stream would not be waited for by a caller's non-blocking stream, and blocks
+  // from the pool hold another handle's values.
+  template <typename T>
+  int zero(T* p, size_t count) {
+    LUB_CUDA(cudaMemsetAsync(p, 0, count * sizeof(T), sG));
+    LUB_CUDA(cudaStreamSynchronize(sG));
+    return LU_OK;
+  }
   void release(void* p) {
     if (!p) return;
     cudaFree(p);

@@ -72,7 +72,7 @@ int ensure_mixed(lu_handle h) {
   LUB_TRY(h->alloc(&h->xbest, n));
   LUB_TRY(h->alloc(&h->rbest, n));
   LUB_TRY(h->alloc(&h->racc_best, 1));
-  LUB_CUDA(cudaMemset(h->zero64, 0, sizeof(double) * n));
+  LUB_TRY(h->zero(h->zero64, n));
   h->mixed_ready = true;
   return LU_OK;
 }
@@ -863,7 +863,7 @@ int ensure_multi(lu_handle h) {
   LUB_TRY(h->alloc(&h->mr_Xbest, n * 16));
   LUB_TRY(h->alloc(&h->mr_Rbest, n * 16));
   LUB_TRY(h->alloc(&h->mr_acc, kMultiAccWords));
-  LUB_CUDA(cudaMemset(h->mr_S, 0, sizeof(double) * n * 16));
+  LUB_TRY(h->zero(h->mr_S, n * 16));
   return LU_OK;
 }
 

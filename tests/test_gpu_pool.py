@@ -64,3 +64,35 @@ def test_threads_with_their_own_streams(cuda_dev):
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("n", [700, 1001])
+def test_zeroed_blocks_do_not_wait_for_the_default_stream(cuda_dev, n):
+    """GMRES multiplies against a vector of zeros, which may be another handle's
+    block; it has to be zero on a non-blocking stream too, with the default
+    stream busy."""
+    import charmlu_b200 as lu
+
+    def solve(stream):
+        s = lu.LUSolver(lu.LUConfig(n, 64, precision=lu.LU_PREC_FP16X3, ir_mode=lu.LU_IR_GMRES))
+        x, info = s.refine_solve(A, b, stream=stream)
+        return s, x, info
+
+    A, b, ref = _system(n, n)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    s, _, _ = solve(stream)
+    s.close()
+    # takes two of the blocks and hands them back behind the others, so that the
+    # next handle's vectors are not the ones they were
+    W, x = torch.nn.functional.pad(A, (0, n & 1))[:, :n], b.clone()  # a copy with rows on 16 bytes
+    s = lu.LUSolver(lu.LUConfig(n, 64))
+    s.factor_solve(W, x)
+    s.close()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(int(5e8))  # about a quarter of a second
+    s, x, info = solve(stream)
+    torch.cuda.synchronize()
+    assert info["status"] == 0 and info["used_gmres"] == 1
+    assert np.abs(x.cpu().numpy() - ref).max() <= 1e-10 * np.abs(ref).max()
+    s.close()
