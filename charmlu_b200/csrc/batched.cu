@@ -80,7 +80,72 @@ struct WorkHeader {
 };
 static_assert(sizeof(WorkHeader) <= 256, "workspace header exceeds its 256 bytes");
 
-__device__ __forceinline__ void tuning_for(int n, int esize, int& nb, int& small) {
+// Outer block width of the two-level blocking: the inner panels (nb columns)
+// are brought up to date inside the outer block as they come up; the rest of
+// the trailing matrix gets one update of depth outer_block per outer block.
+template <typename T>
+constexpr int outer_block() { return sizeof(T) == 8 ? 64 : 128; }
+
+// Dynamic shared memory of factor_system at the panel of columns k0 .. k0 + kw,
+// in elements of T: U rows of the outer block's earlier panels from 0 (pitch
+// up), the panel (kw columns of pitch mp) at lb, then the panel kernel's rows.
+// Before the panel takes its place, L of the earlier panels lies at lb; while it
+// is loaded, FP32 stages stage_rows rows of L (pitch kStagePitch) behind it.
+// Every pointer of factor_system comes from here, and end is the last element
+// that any of them reaches.
+constexpr int kStagePitch = 33, kStageMin = 64;
+template <typename T>
+struct PanelLayout {
+  int Kp, kw, m, mp, up, W, lb, rowbuf, urow, zero, stage, stage_rows, end;
+  __host__ __device__ PanelLayout(int n, int nb, int k0) {
+    constexpr bool f64 = sizeof(T) == 8;
+    Kp = k0 % outer_block<T>();
+    m = n - k0;
+    kw = nb < m ? nb : m;
+    mp = m | 1;
+    up = f64 ? kw + 2 : kw;
+    W = kw <= 8 && f64 ? 8 : (kw <= 16 ? 16 : 32);
+    lb = (Kp * up + 3) & ~3;
+    rowbuf = lb + ((kw * mp + 3) & ~3);
+    urow = rowbuf + (f64 ? 0 : 2 * NWARP * W);
+    zero = urow + W * W;
+    end = zero + W;
+    stage = rowbuf;
+    stage_rows = 0;
+    if (Kp > 0) {
+      const int lt = lb + Kp * (Kp + 4);
+      if (lt > end) end = lt;
+      if (!f64) {
+        // 256 rows, or as many as there is room for
+        stage_rows = ((int)(kBatchSmem / sizeof(T)) - stage) / kStagePitch;
+        if (stage_rows > 256) stage_rows = 256;
+        if (stage_rows < kStageMin) stage_rows = kStageMin;
+        if (stage + stage_rows * kStagePitch > end) end = stage + stage_rows * kStagePitch;
+      }
+    }
+  }
+};
+
+// Panel width for order n, at most nb.  The first sum sets the orders at which
+// the width halves (a panel and 128 columns of it; another line would change the
+// order of the sums, and with it the last bits).  The second is what a panel
+// needs at least, an upper bound of PanelLayout::end with kStageMin staged rows.
+template <typename T>
+__host__ __device__ inline int panel_width(int n, int nb) {
+  constexpr int NB = outer_block<T>();
+  constexpr int cap = (int)(kBatchSmem / sizeof(T));
+  while (nb > 4) {
+    const int W = nb <= 16 ? 16 : 32, rows = 2 * NWARP * W + W * W + W;
+    const int tail = sizeof(T) == 4 && rows < kStageMin * kStagePitch ? kStageMin * kStagePitch : rows;
+    if (n * (nb + 1) + nb * 128 <= cap && 2 * NB + nb * (n + 1) + 8 + tail <= cap) break;
+    nb >>= 1;
+  }
+  return nb;
+}
+
+template <typename T>
+__device__ __forceinline__ void tuning_for(int n, int& nb, int& small) {
+  constexpr int esize = (int)sizeof(T);
   nb = esize == 8 ? 16 : 32;
   small = esize == 8 ? 128 : 192;
   for (int i = 0; i < c_tuning_n; i++) {
@@ -90,18 +155,10 @@ __device__ __forceinline__ void tuning_for(int n, int esize, int& nb, int& small
       break;
     }
   }
-  // shared-memory caps: small path n x (n+1); blocked path panel m x (nb+1) + nb x 128 staging
+  // the small path holds n x (n | 1) elements
   const int small_cap = (int)(sqrtf((float)(kBatchSmem / esize)) - 1.f);
   if (small > small_cap) small = small_cap;
-  // the update phase reuses the same space: a U slice and two L tiles of
-  // depth up to the outer block width
-  const size_t ob = esize == 8 ? 64 : 128;
-  while (nb > 4) {
-    const size_t panel_phase = (size_t)n * (nb + 1) + (size_t)nb * 128;
-    const size_t update_phase = ob * 128 + (size_t)2 * 64 * ob;
-    if ((panel_phase > update_phase ? panel_phase : update_phase) * esize <= kBatchSmem) break;
-    nb >>= 1;
-  }
+  nb = panel_width<T>(n, nb);
 }
 
 // Element copy global -> shared through the async copy unit; pred false
@@ -115,12 +172,6 @@ __device__ __forceinline__ void cp_async_elem(void* sdst, const void* gsrc, bool
 __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Outer block width of the two-level blocking: the inner panels (nb columns)
-// are brought up to date inside the outer block as they come up; the rest of
-// the trailing matrix gets one update of depth kOuter per outer block.
-template <typename T>
-constexpr int outer_block() { return sizeof(T) == 8 ? 64 : 128; }
 
 // Shared memory beside the dynamic part.  Row numbers of one system fit 16 bits.
 template <typename T>
@@ -408,7 +459,7 @@ __device__ __forceinline__ void copy_panel(const T* A, int n, int k0, int kw, in
 // earlier panels (columns K0 .. k0 of L, U rows at ut, pitch up): per nb of
 // them the products are summed from zero, then subtracted.
 __device__ __forceinline__ void load_panel(const double* A, int n, int k0, int kw, int m, int K0, int nb, double* lb,
-                                           int mp, const double* ut, int up) {
+                                           int mp, const double* ut, int up, double*, int) {
   const int tid = threadIdx.x, Kp = k0 - K0;
   if (Kp == 0) {
     copy_panel(A, n, k0, kw, m, lb, mp);
@@ -473,28 +524,28 @@ __device__ __forceinline__ void load_panel(const double* A, int n, int k0, int k
   }
 }
 __device__ __forceinline__ void load_panel(const float* A, int n, int k0, int kw, int m, int K0, int nb, float* lb,
-                                           int mp, const float* ut, int up) {
+                                           int mp, const float* ut, int up, float* ls, int stage_rows) {
   const int tid = threadIdx.x, Kp = k0 - K0;
   copy_panel(A, n, k0, kw, m, lb, mp);
   if (Kp == 0) return;
   __syncthreads();
-  // 256 rows of L (nb columns) at a time through shared memory, one row and
-  // 16 of the panel's columns per thread, U broadcast
-  float* ls = lb + ((kw * mp + 3) & ~3);  // [256][33]
+  // up to 256 rows of L (nb columns) at a time through shared memory, one row
+  // and 16 of the panel's columns per thread, U broadcast
   const int lg = 31 - __clz(nb), row = tid & 255, cb = (tid >> 8) * 16;
   for (int q = 0; q < Kp; q += nb) {
-    for (int r0 = 0; r0 < m; r0 += 256) {
-      for (int idx = tid; idx < (256 << lg); idx += BT) {
+    for (int r0 = 0; r0 < m; r0 += stage_rows) {
+      const int nr = min(stage_rows, m - r0);
+      for (int idx = tid; idx < (nr << lg); idx += BT) {
         const int i = idx >> lg, k = idx & (nb - 1);
-        if (r0 + i < m) cp_async_elem<4>(ls + i * 33 + k, A + (int64_t)(k0 + r0 + i) * n + K0 + q + k, true);
+        cp_async_elem<4>(ls + i * kStagePitch + k, A + (int64_t)(k0 + r0 + i) * n + K0 + q + k, true);
       }
       cp_async_commit_group();
       cp_async_wait_group<0>();
       __syncthreads();
-      if (r0 + row < m && cb < kw) {
+      if (row < nr && cb < kw) {
         float acc[16] = {};
         for (int k = 0; k < nb; k++) {
-          const float l = ls[row * 33 + k];
+          const float l = ls[row * kStagePitch + k];
           const float* ur = ut + (q + k) * up + cb;
           if (kw % 16 == 0) {
 #pragma unroll
@@ -856,21 +907,21 @@ template <typename T>
 __device__ int factor_system(T* A, int n, unsigned char* smem, BShared<T>& sh) {
   const int tid = threadIdx.x;
   int nb, small;
-  tuning_for(n, (int)sizeof(T), nb, small);
+  tuning_for<T>(n, nb, small);
   for (int i = tid; i < n; i += BT) sh.perm[i] = (unsigned short)i;
   if (n <= small) return factor_small<T>(A, n, smem, sh);
   constexpr int NB = outer_block<T>();
   T* ut = reinterpret_cast<T*>(smem);
   int info = 0;
   for (int k0 = 0; k0 < n; k0 += nb) {
-    const int kw = min(nb, n - k0), m = n - k0, mp = m | 1, c1 = k0 + kw;
-    const int K0 = k0 - k0 % NB, Kend = min(n, K0 + NB), Kp = k0 - K0;
-    const int up = sizeof(T) == 8 ? kw + 2 : kw;
-    const int W = kw <= 8 && sizeof(T) == 8 ? 8 : (kw <= 16 ? 16 : 32);
-    T* lb = ut + ((Kp * up + 3) & ~3);  // [kw][mp]
-    T* rowbuf = lb + ((kw * mp + 3) & ~3);
-    T* urow = rowbuf + (sizeof(T) == 4 ? 2 * NWARP * W : 0);
-    T* zero = urow + W * W;
+    const PanelLayout<T> lay(n, nb, k0);
+    const int kw = lay.kw, m = lay.m, mp = lay.mp, c1 = k0 + kw;
+    const int Kp = lay.Kp, K0 = k0 - Kp, Kend = min(n, K0 + NB);
+    const int up = lay.up, W = lay.W;
+    T* lb = ut + lay.lb;  // [kw][mp]
+    T* rowbuf = ut + lay.rowbuf;
+    T* urow = ut + lay.urow;
+    T* zero = ut + lay.zero;
     if (Kp == 0)
       for (int i = tid; i < n - K0; i += BT) sh.ob[i] = (unsigned short)i;
     if (Kp > 0) {
@@ -891,7 +942,7 @@ __device__ int factor_system(T* A, int n, unsigned char* smem, BShared<T>& sh) {
         if (c < kw) A[(int64_t)(K0 + i) * n + k0 + c] = ut[i * up + c];
       }
     }
-    load_panel(A, n, k0, kw, m, K0, nb, lb, mp, ut, up);
+    load_panel(A, n, k0, kw, m, K0, nb, lb, mp, ut, up, ut + lay.stage, lay.stage_rows);
     __syncthreads();
     int pi;
     if (W == 8) {
@@ -1323,6 +1374,30 @@ extern "C" LU_API int lu_batched_set_tuning(int32_t entries, const int32_t* tabl
   LUB_CUDA(cudaMemcpyToSymbol(c_tuning, t, sizeof(t)));
   LUB_CUDA(cudaMemcpyToSymbol(c_tuning_n, &entries, sizeof(int)));
   return LU_OK;
+}
+
+namespace {
+template <typename T>
+int layout_probe(int n, int nb, int* out) {
+  nb = panel_width<T>(n, nb);
+  out[0] = nb;
+  out[1] = 0;
+  out[2] = 256;
+  for (int k0 = 0; k0 < n; k0 += nb) {
+    const PanelLayout<T> lay(n, nb, k0);
+    out[1] = std::max(out[1], lay.end * (int)sizeof(T));
+    if (lay.stage_rows > 0) out[2] = std::min(out[2], lay.stage_rows);
+  }
+  return LU_OK;
+}
+}  // namespace
+
+// Test hook (no GPU): out = panel width taken for order n where the table says
+// nb, bytes of dynamic shared memory that its panels reach, fewest staged rows
+// of L, bytes that the kernel asks for.
+extern "C" __attribute__((visibility("default"))) int lub_test_batched_layout(int n, int nb, int esize, int* out) {
+  out[3] = (int)kBatchSmem;
+  return esize == 8 ? layout_probe<double>(n, nb, out) : layout_probe<float>(n, nb, out);
 }
 
 extern "C" LU_API int lu_batched_factor_solve(int32_t count, const int32_t* n, const int64_t* a_off,

@@ -195,3 +195,21 @@ def test_batched_singular_and_ties(cuda_dev):
     assert info.tolist() == [n // 2 + 1 for n in ns] + [0] * 4
     o = int(bs.b_off[4])
     np.testing.assert_array_equal(b.cpu().numpy()[o:], rhs[o:])
+
+
+@pytest.mark.parametrize("prec", [LU_PREC_FP64, LU_PREC_FP32])
+@pytest.mark.parametrize("orders", [[1335, 1336, 1400, 1427], [1385, 1386, 1428, 1536], [1537, 2047, 2048]])
+def test_batched_orders_above_1025(cuda_dev, prec, orders):
+    """Orders around those at which the panel width halves (FP64 1386, FP32 1428),
+    at which fewer rows of L are staged (FP32 1336 .. 1427), and the largest;
+    several panels of 512 rows per thread.  The contract of every system."""
+    n = np.array(orders, dtype=np.int32)
+    a_off = np.concatenate([[0], np.cumsum(n.astype(np.int64) ** 2)[:-1]]).astype(np.int64)
+    b_off = np.concatenate([[0], np.cumsum(n.astype(np.int64))[:-1]]).astype(np.int64)
+    A0, b0, x, info, _ = _run(n, a_off, b_off, prec, seed=int(n[0]))
+    assert np.all(info == 0), info
+    eps = np.finfo(np.float64).eps
+    for i, k in enumerate(orders):
+        Ai, bi, xi = A0[a_off[i]:a_off[i] + k * k].reshape(k, k), b0[b_off[i]:b_off[i] + k], x[b_off[i]:b_off[i] + k]
+        scale = np.abs(Ai).sum(1).max() * np.abs(xi).max() + np.abs(bi).max()
+        assert np.abs(bi - Ai @ xi).max() < 16 * k * eps * scale, k
