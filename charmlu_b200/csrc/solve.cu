@@ -371,12 +371,11 @@ __device__ void tri_inverse_tile(const TD* D, int ldd, TI* Dinv, int ldi, int ro
   }
 }
 
-// Pipeline progress: CTAs finish in ticket order (each waits for its
-// predecessor), so one counter, set to ticket + 1 when a CTA has published
-// its rows, tells every later CTA how many blocks are final.  A waiter far
-// behind the front sleeps in proportion to its distance, which keeps the
-// polls on that one word sparse.  Bounded: false after `spin` polls or when
-// another CTA has recorded an error.
+// Pipeline progress: one counter, set to ticket + 1 when a CTA has published
+// its rows and every CTA before it has (publish_progress), tells every later
+// CTA how many blocks are final.  A waiter far behind the front sleeps in
+// proportion to its distance, which keeps the polls on that one word sparse.
+// Bounded: false after `spin` polls or when another CTA has recorded an error.
 __device__ __forceinline__ bool wait_progress(const int* counter, int need, int* seen, DevStatus* st, long long spin,
                                               int where) {
   long long polls = 0;
@@ -390,6 +389,18 @@ __device__ __forceinline__ bool wait_progress(const int* counter, int need, int*
   }
   *seen = v;
   return true;
+}
+
+// Block tk's rows are in memory (stored by the CTA, then a CTA barrier): sets the
+// counter to tk + 1, once it stands at tk.  The packets below let block tk + 1
+// finish before block tk gets here.  Stored out of turn, the counter would go
+// backwards, and who acquires tk + 2 could read block tk's rows before they are
+// there; in turn, every store of the counter follows the rows of all blocks up
+// to its value.  The packets have left by now, so this is not on the chain.
+// Called by one thread; bounded as wait_progress.
+__device__ __forceinline__ void publish_progress(int* counter, int tk, DevStatus* st, long long spin, int where) {
+  int v;
+  if (wait_progress(counter, tk, &v, st, spin, where)) st_release_s32(counter, tk + 1);
 }
 
 // A finished block's rows also leave as 16-byte packets {value, tag} in a ring
@@ -578,7 +589,7 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TS* LU, int64_t lda, in
   // CTA barrier, then thread 0's release store: the rows written above are
   // visible to every CTA that acquires the counter
   __syncthreads();
-  if (tid == 0) st_release_s32(&flags[0], tk + 1);
+  if (tid == 0) publish_progress(&flags[0], tk, st, spin, 301);
 }
 
 // ---------------------------------------------------------------------------
@@ -798,7 +809,7 @@ __global__ void __launch_bounds__(256, 2) trsm_pipe_kernel(const TS* LU, int64_t
   // CTA barrier, then thread 0's release store: the rows written above are
   // visible to every CTA that acquires the counter
   __syncthreads();
-  if (tid == 0) st_release_s32(progress, tk + 1);
+  if (tid == 0) publish_progress(progress, tk, st, spin, 302);
 }
 
 // G = -Lam * X^T (n x n), Lam and X n x k row-major, k <= 16: the rank-k
@@ -1052,4 +1063,55 @@ extern "C" __attribute__((visibility("default"))) int lub_test_trsm_wide(const f
   cudaStreamSynchronize((cudaStream_t)stream);
   cudaFree(dinv);
   return rc;
+}
+
+
+// Test hook: one CTA, warp w publishes block tickets - 1 - w, the later blocks
+// first in time; one more warp watches the counter.  out: [0] the counter at the
+// end, [1] times it went backwards, [2] blocks it named whose row was not there
+// yet, [3] the status code.  rows: 16 zeroed ints.  tickets <= 16.
+namespace lub {
+namespace {
+__global__ void publish_progress_test_kernel(int* counter, int* rows, int tickets, DevStatus* st, int* out) {
+  const int warp = threadIdx.x >> 5;
+  if (threadIdx.x & 31) return;
+  if (warp < tickets) {
+    const int tk = tickets - 1 - warp;
+    for (int i = 0; i < 20 * (warp + 1); i++) __nanosleep(1000);
+    *(volatile int*)&rows[tk] = 1;
+    publish_progress(counter, tk, st, 1LL << 20, 301);
+  } else {
+    int last = 0, back = 0, early = 0;
+    for (int polls = 0; polls < (1 << 20) && last < tickets; polls++) {
+      const int v = ld_acquire_s32(counter);
+      if (v < last) back++;
+      if (v > last)
+        for (int q = 0; q < v; q++)
+          if (*(volatile int*)&rows[q] == 0) early++;
+      last = v;
+    }
+    out[1] = back;
+    out[2] = early;
+  }
+}
+}  // namespace
+}  // namespace lub
+extern "C" __attribute__((visibility("default"))) int lub_test_publish_progress(int tickets, int* scratch, int* out,
+                                                                                void* stream) {
+  using namespace lub;
+  if (tickets < 1 || tickets > 16) return LU_ERR_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  // scratch: 32 ints on the device; [0] counter, [4, 8) status, [8, 24) rows, [24, 28) out
+  LUB_CUDA(cudaMemsetAsync(scratch, 0, 32 * sizeof(int), s));
+  DevStatus* st = reinterpret_cast<DevStatus*>(scratch + 4);
+  publish_progress_test_kernel<<<1, 32 * (tickets + 1), 0, s>>>(scratch, scratch + 8, tickets, st, scratch + 24);
+  LUB_LAUNCH_CHECK();
+  int h[32];
+  LUB_CUDA(cudaMemcpyAsync(h, scratch, sizeof(h), cudaMemcpyDeviceToHost, s));
+  LUB_CUDA(cudaStreamSynchronize(s));
+  out[0] = h[0];
+  out[1] = h[25];
+  out[2] = h[26];
+  out[3] = h[4];
+  return LU_OK;
 }
