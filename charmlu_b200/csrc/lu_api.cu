@@ -368,7 +368,7 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
   if (s == LU_OK) s = h->alloc(&h->vec, n);
   if (s == LU_OK) s = h->alloc(&h->vec2, n);
   if (s == LU_OK) s = h->alloc(&h->racc, 1);
-  if (s == LU_OK && cudaMemset(h->st, 0, sizeof(DevStatus)) != cudaSuccess) s = LU_ERR_CUDA;
+  if (s == LU_OK) s = h->zero(h->st, 1);
   if (s != LU_OK) {
     lu_destroy(h);
     return s;

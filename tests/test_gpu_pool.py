@@ -96,3 +96,29 @@ def test_zeroed_blocks_do_not_wait_for_the_default_stream(cuda_dev, n):
     assert info["status"] == 0 and info["used_gmres"] == 1
     assert np.abs(x.cpu().numpy() - ref).max() <= 1e-10 * np.abs(ref).max()
     s.close()
+
+
+def _singular_factor(n, stream):
+    """A handle whose status word holds a singular column; the stream has finished."""
+    import charmlu_b200 as lu
+    A = torch.zeros(n, n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    s = lu.LUSolver(lu.LUConfig(n, 64))
+    s.factor(A, stream=stream)
+    assert s.status(stream) == 1
+    return s
+
+
+def test_a_status_outlives_the_default_streams_work(cuda_dev):
+    """Nothing that lu_create left on the default stream clears a later status."""
+    stream = torch.cuda.Stream()
+    _singular_factor(256, stream).close()
+    A = torch.zeros(256, 256, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    import charmlu_b200 as lu
+    torch.cuda._sleep(int(5e8))
+    s = lu.LUSolver(lu.LUConfig(256, 64))
+    s.factor(A, stream=stream)
+    torch.cuda.synchronize()
+    assert s.status(stream) == 1
+    s.close()
