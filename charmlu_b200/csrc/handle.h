@@ -43,6 +43,8 @@ struct HandleRes {
   void* pinned = nullptr;                   // sizeof(ResidualAccum)
 };
 int pool_alloc(void** p, size_t bytes, size_t* got);
+// a new block of the caller's own, for cudaFree
+int pool_malloc(void** p, size_t bytes);
 // p must not be in use by the device any more
 void pool_free(int device, void* p, size_t bytes);
 int pool_take_res(HandleRes* r);

@@ -316,7 +316,8 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
   // one per leaf launch (leaves are >= 2 columns wide) and one per shared
   // trailing-update tile counter (panels are >= 64 columns wide)
   h->n_counters = (int)(n / 2 + n / 64 + 1024);
-  if (s == LU_OK) s = h->alloc(&h->st, 1);
+  // never from the pool: freeing it is what lu_destroy waits by
+  if (s == LU_OK) s = pool_malloc((void**)&h->st, sizeof(DevStatus));
   if (s == LU_OK) s = h->alloc(&h->leaf_pkt, kLeafPackets + (h->n_counters + 3) / 4);
   h->counters = reinterpret_cast<unsigned*>(h->leaf_pkt + kLeafPackets);
   if (s == LU_OK) s = h->alloc(&h->plist.dst, 2 * kMaxBatch);
@@ -387,11 +388,14 @@ int lu_destroy(lu_handle h) {
     if (h->evFree[b]) cudaEventDestroy(h->evFree[b]);
   }
   if (h->sCopy) cudaStreamDestroy(h->sCopy);
-  // the handle's work may still run: wait as the frees would, on its device
+  // The handle's work may still run: wait for it, on its device, before the pool
+  // takes the blocks.  cudaFree waits for every stream; cudaDeviceSynchronize does
+  // too, but it ends any capture of this process in an error, also one of
+  // another thread (lu_factor of a handle with use_graph is one).
   int cur = h->device;
   cudaGetDevice(&cur);
   if (cur != h->device) cudaSetDevice(h->device);
-  const bool idle = cudaDeviceSynchronize() == cudaSuccess;
+  const bool idle = cudaFree(h->st) == cudaSuccess;
   if (!idle) cudaGetLastError();
   for (auto& blk : h->allocs) {
     if (idle) pool_free(h->device, blk.first, blk.second);

@@ -32,6 +32,17 @@ void drop(DevPool& d, size_t i) {
   d.blocks.erase(d.blocks.begin() + i);
 }
 
+// cudaMalloc, after giving the cached blocks back if there is no room (lock held)
+int malloc_or_empty(DevPool& d, void** p, size_t bytes) {
+  if (cudaMalloc(p, bytes) == cudaSuccess) return LU_OK;
+  cudaGetLastError();
+  while (!d.blocks.empty()) drop(d, d.blocks.size() - 1);
+  if (cudaMalloc(p, bytes) == cudaSuccess) return LU_OK;
+  cudaGetLastError();
+  *p = nullptr;
+  return LU_ERR_NOMEM;
+}
+
 void destroy_res(const HandleRes& r) {
   if (r.sP) cudaStreamDestroy(r.sP);
   if (r.sG) cudaStreamDestroy(r.sG);
@@ -71,12 +82,15 @@ int pool_alloc(void** p, size_t bytes, size_t* got) {
     return LU_OK;
   }
   *got = want;
-  if (cudaMalloc(p, want) == cudaSuccess) return LU_OK;
-  cudaGetLastError();
-  while (!d.blocks.empty()) drop(d, d.blocks.size() - 1);
-  if (cudaMalloc(p, want) == cudaSuccess) return LU_OK;
-  cudaGetLastError();
-  return LU_ERR_NOMEM;
+  return malloc_or_empty(d, p, want);
+}
+
+int pool_malloc(void** p, size_t bytes) {
+  int dev = 0;
+  LUB_TRY(current_device(&dev));
+  DevPool& d = pool_of(dev);
+  std::lock_guard<std::mutex> lk(d.mu);
+  return malloc_or_empty(d, p, bytes);
 }
 
 void pool_free(int device, void* p, size_t bytes) {

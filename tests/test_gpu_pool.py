@@ -122,3 +122,87 @@ def test_a_status_outlives_the_default_streams_work(cuda_dev):
     torch.cuda.synchronize()
     assert s.status(stream) == 1
     s.close()
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
+def test_a_handle_goes_beside_a_capture(cuda_dev, mode):
+    """Destroying a handle leaves a capture alone: another thread's, and in relaxed
+    mode this thread's."""
+    import charmlu_b200 as lu
+    n = 256
+    s = lu.LUSolver(lu.LUConfig(n, 64))
+    s.factor(torch.rand(n, n, dtype=torch.float64, device="cuda"))
+    assert s.status() == 0
+    y = torch.ones(64, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode=mode):
+        x = y * 2
+        if mode == "relaxed":
+            s.close()
+        else:
+            t = threading.Thread(target=s.close)
+            t.start()
+            t.join()
+        z = x + 1
+    g.replay()
+    assert torch.equal(z, torch.full_like(z, 3.0))
+
+
+def test_handles_come_and_go_beside_graph_schedules(cuda_dev):
+    """One thread's solver captures its schedule anew for every matrix while
+    another thread makes and destroys handles."""
+    import charmlu_b200 as lu
+    bad, done = [], threading.Event()
+
+    def schedules():
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                s = lu.LUSolver(lu.LUConfig(1024, 128, use_graph=True))
+                keep = []
+                for it in range(30):
+                    A = torch.rand(1024, 1024, dtype=torch.float64, device="cuda")
+                    keep.append(A)  # another address, so another capture
+                    s.factor(A, stream=stream)
+                    if s.status(stream) != 0:
+                        bad.append(("status", it))
+                s.close()
+        except Exception as e:  # reported by the main thread
+            bad.append(("schedules", repr(e)))
+        done.set()
+
+    def handles():
+        try:
+            stream = torch.cuda.Stream()
+            with torch.cuda.stream(stream):
+                A = torch.rand(256, 256, dtype=torch.float64, device="cuda")
+                while not done.is_set():
+                    s = lu.LUSolver(lu.LUConfig(256, 64))
+                    s.factor(A.clone(), stream=stream)
+                    if s.status(stream) != 0:
+                        bad.append("status of a short-lived handle")
+                    s.close()
+        except Exception as e:
+            bad.append(("handles", repr(e)))
+
+    threads = [threading.Thread(target=f) for f in (schedules, handles)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+
+
+def test_destroy_waits_for_the_handles_work(cuda_dev):
+    import charmlu_b200 as lu
+    n = 256
+    stream = torch.cuda.Stream()
+    A = torch.rand(n, n, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(3):
+        s = lu.LUSolver(lu.LUConfig(n, 64))
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(int(2e8))  # about a tenth of a second
+            s.factor(A, stream=stream)
+        s.close()
+        assert stream.query()
