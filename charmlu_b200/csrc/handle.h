@@ -181,6 +181,7 @@ struct lu_handle_s {
   std::vector<std::pair<void*, size_t>> allocs;  // block, its size in the pool
   lub::HandleRes res;
   size_t bytes = 0;
+  bool created = false;  // lu_create has returned
   long long spin = 0;
   // CUDA-graph replay of factorisation schedules (cfg.use_graph)
   struct GraphSlot {
@@ -223,6 +224,18 @@ struct lu_handle_s {
   int alloc(T** p, size_t count) {
     void* q = nullptr;
     size_t got = 0;
+    // cudaMalloc is refused while this thread captures (unless in relaxed mode).
+    // A block from the pool would not be: what grows on a first call asks by a
+    // query that is refused then too, so that the same calls are refused
+    // whatever the pool holds.  (lu_create allocates its status word first.)
+    if (created) {
+      const cudaError_t e = cudaStreamQuery(sG);
+      if (e != cudaSuccess && e != cudaErrorNotReady) {
+        cudaGetLastError();
+        return LU_ERR_NOMEM;
+      }
+      cudaGetLastError();  // NotReady is not kept
+    }
     if (int rc = lub::pool_alloc(&q, count * sizeof(T), &got)) return rc;
     allocs.emplace_back(q, got);
     bytes += count * sizeof(T);

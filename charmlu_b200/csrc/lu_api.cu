@@ -370,6 +370,7 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
   if (s == LU_OK) s = h->alloc(&h->vec2, n);
   if (s == LU_OK) s = h->alloc(&h->racc, 1);
   if (s == LU_OK) s = h->zero(h->st, 1);
+  h->created = s == LU_OK;
   if (s != LU_OK) {
     lu_destroy(h);
     return s;

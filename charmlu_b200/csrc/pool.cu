@@ -26,18 +26,25 @@ DevPool& pool_of(int dev) {
   return pools[dev];
 }
 
+// a block that cannot be freed now (during a capture, say) stays
 void drop(DevPool& d, size_t i) {
-  cudaFree(d.blocks[i].p);
+  if (cudaFree(d.blocks[i].p) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
   d.cached -= d.blocks[i].bytes;
   d.blocks.erase(d.blocks.begin() + i);
 }
 
 // cudaMalloc, after giving the cached blocks back if there is no room (lock held)
 int malloc_or_empty(DevPool& d, void** p, size_t bytes) {
-  if (cudaMalloc(p, bytes) == cudaSuccess) return LU_OK;
-  cudaGetLastError();
-  while (!d.blocks.empty()) drop(d, d.blocks.size() - 1);
-  if (cudaMalloc(p, bytes) == cudaSuccess) return LU_OK;
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    for (size_t i = d.blocks.size(); i-- > 0;) drop(d, i);
+    e = cudaMalloc(p, bytes);
+  }
+  if (e == cudaSuccess) return LU_OK;
   cudaGetLastError();
   *p = nullptr;
   return LU_ERR_NOMEM;

@@ -1,5 +1,6 @@
 """Handles made from what earlier ones left (device blocks, streams, events):
 blocks with another order's leftovers, several threads and streams at once."""
+import ctypes
 import threading
 
 import numpy as np
@@ -206,3 +207,41 @@ def test_destroy_waits_for_the_handles_work(cuda_dev):
             s.factor(A, stream=stream)
         s.close()
         assert stream.query()
+
+
+@pytest.mark.parametrize("pooled", [False, True])
+def test_handles_are_not_made_inside_a_capture(cuda_dev, pooled):
+    """Refused while the calling thread captures, whatever earlier handles left
+    behind; so are blocks that an existing handle lacks."""
+    import charmlu_b200 as lu
+    n = 320
+    rt = ctypes.CDLL(next(ln.split()[-1] for ln in open("/proc/self/maps") if "libcudart" in ln))
+    A, B = torch.rand(n, n, dtype=torch.float64, device="cuda"), torch.rand(n, 8, dtype=torch.float64, device="cuda")
+    first, kept = lu.LUSolver(lu.LUConfig(n, 64)), lu.LUSolver(lu.LUConfig(n, 64))
+    piv = first.factor(A)
+    first.solve(A, piv, B.clone())
+    assert first.status() == 0
+    if pooled:
+        first.close()
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+
+    def refused(call):
+        sp, graph = ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p()
+        assert rt.cudaStreamBeginCapture(sp, 1) == 0  # thread-local mode
+        try:
+            with pytest.raises(lu.LUError):
+                call()
+        finally:
+            rt.cudaStreamEndCapture(sp, ctypes.byref(graph))
+            rt.cudaGetLastError()
+
+    refused(lambda: lu.LUSolver(lu.LUConfig(n, 64)))
+    refused(lambda: kept.solve(A, piv, B.clone(), stream=stream))
+    # both work afterwards
+    X = B.clone()
+    kept.solve(A, piv, X)
+    assert kept.status() == 0
+    lu.LUSolver(lu.LUConfig(n, 64)).close()
+    kept.close()
+    first.close()
