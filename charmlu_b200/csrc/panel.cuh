@@ -608,14 +608,59 @@ int max_cluster() {
   return n >= 1 ? kMaxCluster : 8;
 }
 
+// Rows per thread of the grid and cluster instances (launch_leaf_w); 8 columns
+// wide there is one grid instance of twice as many rows
+template <typename T, int W>
+constexpr int leaf_rows() { return max_rpt<T, W>() < 6 ? max_rpt<T, W>() : 6; }
+constexpr int kTallRows = 12;
+
+inline int leaf_cta_limit(int num_sms) { return std::min(num_sms, kMaxLeafCTAs); }
+
+struct LeafPlan {
+  int W, xp, G, R, rpt;  // instance, transport, CTAs, rows per CTA and per thread
+};
+// One CTA up to 512 rows (two per thread: no exchange at all); alone on the GPU
+// (cluster > 0 CTAs in the largest cluster) one cluster, one row per thread
+// first, then more CTAs, then more rows; else a cooperative grid, one CTA per
+// SM, of at most max_ctas CTAs (more only when the rows need their registers).
+template <typename T>
+int leaf_plan(int M, int ncols, int num_sms, int max_ctas, int cluster, LeafPlan* p) {
+  const int limit = leaf_cta_limit(num_sms);
+  p->W = ncols <= 16 ? 16 : 32;
+  const int rmax = p->W == 16 ? leaf_rows<T, 16>() : leaf_rows<T, 32>();
+  p->G = 1;
+  p->xp = kSingle;
+  if (M > 2 * NT) {
+    if (M <= (int64_t)cluster * NT * rmax) {
+      p->xp = kCluster;
+      p->G = 2;
+      while (p->G < cluster && p->G * NT < M) p->G *= 2;
+    } else {
+      p->xp = kGrid;
+      p->G = std::min(ceil_div(M, NT), std::min(max_ctas, limit));
+      p->G = std::max(p->G, ceil_div(M, NT * rmax));
+      if (p->G > limit) {  // twice the rows of half the width
+        if (ncols > 8) return LU_ERR_UNSUPPORTED;
+        p->W = 8;
+        p->G = ceil_div(M, NT * kTallRows);
+        if (p->G > limit) return LU_ERR_UNSUPPORTED;
+      }
+    }
+  }
+  p->R = ceil_div(M, p->G);
+  if (p->xp == kGrid) p->G = ceil_div(M, p->R);
+  p->rpt = p->W == 8 ? kTallRows : ceil_div(p->R, NT);
+  return LU_OK;
+}
+
 }  // namespace
 
 // Narrower than 16 only for panels too tall for the registers of every SM.
 template <typename T>
 int leaf_max_width(int M, int num_sms) {
-  const int64_t rows = (int64_t)std::min(num_sms, kMaxLeafCTAs) * NT;
-  if (M <= rows * max_rpt<T, 32>()) return 32;
-  if (M <= rows * max_rpt<T, 16>()) return 16;
+  const int64_t rows = (int64_t)leaf_cta_limit(num_sms) * NT;
+  if (M <= rows * leaf_rows<T, 32>()) return 32;
+  if (M <= rows * leaf_rows<T, 16>()) return 16;
   return 8;
 }
 
@@ -631,52 +676,26 @@ int launch_getf2_leaf(T* P, int64_t lda, int M, int ncols, int32_t* ipiv, int ro
     lc0 = 0;
   }
   if (lc0 < 0 || lc0 + ncols > pw) return LU_ERR_ARG;
-  static int s_cluster[64];
+  static int s_cluster[64], s_sms[64];
   static PerDeviceOnce once;
   int dev = 0;
   LUB_CUDA(cudaGetDevice(&dev));
   LUB_TRY(once_per_device(once, [&] {
     s_cluster[dev] = max_cluster<T>();
-    return LU_OK;
+    return cuda_status(cudaDeviceGetAttribute(&s_sms[dev], cudaDevAttrMultiProcessorCount, dev));
   }));
-  // Grid: one CTA up to 512 rows (two per thread: no exchange at all); alone
-  // on the GPU one cluster, one row per thread first, then more CTAs, then
-  // more rows; else a cooperative grid of at most max_ctas CTAs (more only
-  // when the rows need their registers).
-  const int w = ncols <= 16 ? 16 : 32;
-  const int rm = w == 16 ? max_rpt<T, 16>() : max_rpt<T, 32>();
-  const int rmax = rm >= 6 ? 6 : rm;
-  int G = 1, xp = kSingle;
-  if (M > 2 * NT) {
-    const int mc = s_cluster[dev];
-    if (alone && M <= (int64_t)mc * NT * rmax) {
-      xp = kCluster;
-      G = 2;
-      while (G < mc && G * NT < M) G *= 2;
-    } else {
-      xp = kGrid;
-      G = std::min(ceil_div(M, NT), std::min(max_ctas, kMaxLeafCTAs));
-      G = std::max(G, ceil_div(M, NT * rmax));
-    }
+  LeafPlan p;
+  LUB_TRY(leaf_plan<T>(M, ncols, s_sms[dev], max_ctas, alone ? s_cluster[dev] : 0, &p));
+  const LeafArgs a{lda, M, ncols, p.R, ipiv, row_base, pkt, tag0, st, info_base, thr, spin, pw, lc0};
+  if (p.W == 8) return launch_leaf<T, 8, kTallRows, kGrid>(P, prow0, a, p.G, s);
+  if (p.W == 16) {
+    if (p.xp == kSingle) return launch_leaf_w<T, 16, kSingle>(P, prow0, a, p.G, p.rpt, s);
+    if (p.xp == kGrid) return launch_leaf_w<T, 16, kGrid>(P, prow0, a, p.G, p.rpt, s);
+    return launch_leaf_w<T, 16, kCluster>(P, prow0, a, p.G, p.rpt, s);
   }
-  int R = ceil_div(M, G), rpt = ceil_div(R, NT);
-  if (xp == kGrid) G = ceil_div(M, R);
-  LeafArgs a{lda, M, ncols, R, ipiv, row_base, pkt, tag0, st, info_base, thr, spin, pw, lc0};
-  if (G > kMaxLeafCTAs) {  // twice the rows of half the width
-    if (ncols > 8) return LU_ERR_UNSUPPORTED;
-    a.R = ceil_div(M, std::max(1, ceil_div(M, NT * 12)));
-    G = ceil_div(M, a.R);
-    if (G > kMaxLeafCTAs) return LU_ERR_UNSUPPORTED;
-    return launch_leaf<T, 8, 12, kGrid>(P, prow0, a, G, s);
-  }
-  if (w == 16) {
-    if (xp == kSingle) return launch_leaf_w<T, 16, kSingle>(P, prow0, a, G, rpt, s);
-    if (xp == kGrid) return launch_leaf_w<T, 16, kGrid>(P, prow0, a, G, rpt, s);
-    return launch_leaf_w<T, 16, kCluster>(P, prow0, a, G, rpt, s);
-  }
-  if (xp == kSingle) return launch_leaf_w<T, 32, kSingle>(P, prow0, a, G, rpt, s);
-  if (xp == kGrid) return launch_leaf_w<T, 32, kGrid>(P, prow0, a, G, rpt, s);
-  return launch_leaf_w<T, 32, kCluster>(P, prow0, a, G, rpt, s);
+  if (p.xp == kSingle) return launch_leaf_w<T, 32, kSingle>(P, prow0, a, p.G, p.rpt, s);
+  if (p.xp == kGrid) return launch_leaf_w<T, 32, kGrid>(P, prow0, a, p.G, p.rpt, s);
+  return launch_leaf_w<T, 32, kCluster>(P, prow0, a, p.G, p.rpt, s);
 }
 
 #define LUB_INSTANTIATE_LEAF(T)                                                                                    \

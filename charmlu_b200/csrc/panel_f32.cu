@@ -26,3 +26,21 @@ extern "C" __attribute__((visibility("default"))) int lub_test_getf2_leaf(float*
   LUB_CUDA(cudaStreamSynchronize(s));
   return rc != LU_OK ? rc : (h.code != 0 ? h.code : h.info);
 }
+
+// Test hook (no GPU): the launch taken for a leaf, out = {widest leaf for M
+// rows, status, instance width, transport, CTAs, rows per CTA, rows per thread}.
+// cluster: CTAs of the largest cluster (0: another kernel runs beside it).
+extern "C" __attribute__((visibility("default"))) int lub_test_leaf_plan(int esize, int M, int ncols, int num_sms,
+                                                                         int max_ctas, int cluster, int* out) {
+  using namespace lub;
+  LeafPlan p{};
+  out[0] = esize == 8 ? leaf_max_width<double>(M, num_sms) : leaf_max_width<float>(M, num_sms);
+  out[1] = esize == 8 ? leaf_plan<double>(M, ncols, num_sms, max_ctas, cluster, &p)
+                      : leaf_plan<float>(M, ncols, num_sms, max_ctas, cluster, &p);
+  out[2] = p.W;
+  out[3] = p.xp;
+  out[4] = p.G;
+  out[5] = p.R;
+  out[6] = p.rpt;
+  return LU_OK;
+}

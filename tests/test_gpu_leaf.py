@@ -127,3 +127,27 @@ def test_ties_zero_and_nonfinite_columns(cuda_dev, M):
         assert rc == first_bad
         assert ipiv.tolist() == want
         np.testing.assert_allclose(A.cpu().numpy(), ref, rtol=0, atol=64 * 2.0 ** -24)
+
+
+@pytest.mark.parametrize("M", [227328, 227329, 240000, 245761])
+def test_panels_taller_than_sixteen_columns_allow(cuda_dev, M):
+    """FP64 panels around 148 CTAs x 6 rows per thread, above which leaves are 8
+    columns wide with 12 rows per thread."""
+    w = 16
+    A0 = torch.rand(M, w, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(M)) - 0.5
+    A = A0.clone()
+    rc, piv = _leaf64(A, w, True)
+    assert rc == 0
+    order = np.arange(M)
+    for j, p in enumerate(piv):
+        assert j <= p < M
+        order[[j, p]] = order[[p, j]]
+    PA = A0[torch.from_numpy(order).cuda()]
+    L = torch.tril(A, -1)
+    L.diagonal().fill_(1.0)
+    U = torch.triu(A[:w])
+    assert L.abs().max() <= 1
+    # w roundings by elimination, as many again in the FP64 products here
+    u = 2.0 ** -53
+    bound = 2 * (w + 1) * u / (1 - 2 * (w + 1) * u) * (L.abs() @ U.abs()) + u
+    assert ((PA - L @ U).abs() <= bound).all()
