@@ -43,6 +43,9 @@ constexpr int kLeafPackets = 2 * kMaxLeafCTAs * (1 + kLeafRowPackets);
 // widest leaf (32, 16 or 8) that num_sms CTAs hold for M rows
 template <typename T>
 int leaf_max_width(int M, int num_sms);
+// CTAs that a leaf of up to 32 columns needs for M rows
+template <typename T>
+int leaf_min_ctas(int M);
 // Factor P[0:M, 0:ncols] (row-major, P = diagonal of the first column, ncols
 // <= 32) with partial pivoting; ipiv[j] = row_base + local pivot row.  Its
 // interchanges are also applied to the enclosing panel's other columns:

@@ -313,6 +313,16 @@ int lowp_gemm(lu_handle h, const CUtensorMap& mapL, const CUtensorMap& mapU, con
   return launch_gemm_bf16_tc(mapL, mapU, mapC, 0, u0, k1, k1 + u0, rest, ncols, K, bf16, amax, h->st, h->spin, s);
 }
 
+// SMs that the update leaves to a panel of M rows beside it: gemm_reserve, or as
+// many CTAs (one per SM, whole CTA pairs) as the panel's leaves need for their
+// rows.  With fewer, a leaf's cooperative grid waits for the end of the update:
+// from 73728 rows with 48 SMs (B200, FP16x3: n = 80000 1315 -> 1280 ms, n = 90000
+// 1845 -> 1740 ms).
+int panel_reserve(int gemm_reserve, int gemm_ctas, int M) {
+  if (gemm_reserve <= 0) return 0;
+  return std::max(gemm_reserve, std::min((leaf_min_ctas<float>(M) + 1) & ~1, gemm_ctas));
+}
+
 // One look-ahead step with the next panel's columns first (pairs layout):
 // on the main stream the interchanges, U solve, operands and update of
 // panel k+1's nw columns; then panel k+1 starts on the panel stream while
@@ -348,15 +358,16 @@ int factor_mixed_split_step(lu_handle h, Ctx32& c, Ctx32& cp, const CUtensorMap&
   CUtensorMap mapL2, mapU2;
   LUB_TRY(build_operands_part(h, c, k0, kw, k1, rest, nw, rest - nw, false, h->amax + 2, &mapL2, &mapU2, &K, &kpart,
                               s));
-  unsigned* ctr = (h->gemm_helper && h->gemm_ctas > 0 && h->gemm_reserve > 0) ? h->take_counter() : nullptr;
+  const int reserve = panel_reserve(h->gemm_reserve, h->gemm_ctas, rest);
+  unsigned* ctr = (h->gemm_helper && h->gemm_ctas > 0 && reserve > 0) ? h->take_counter() : nullptr;
   if (ctr) {
     LUB_CUDA(cudaEventRecord(h->evR, s));
     LUB_CUDA(cudaStreamWaitEvent(h->sP, h->evR, 0));
     LUB_TRY(lowp_gemm(h, mapL2, mapU2, mapC, k1, rest, nw, rest - nw, K, kpart, kw, false, h->sP, 0, ctr,
-                      h->gemm_reserve, h->amax + 2));
+                      reserve, h->amax + 2));
   }
   LUB_CUDA(cudaEventRecord(h->evP, h->sP));
-  return lowp_gemm(h, mapL2, mapU2, mapC, k1, rest, nw, rest - nw, K, kpart, kw, false, s, h->gemm_reserve, ctr, 0,
+  return lowp_gemm(h, mapL2, mapU2, mapC, k1, rest, nw, rest - nw, K, kpart, kw, false, s, reserve, ctr, 0,
                    h->amax + 2);
 }
 
@@ -451,15 +462,14 @@ int factor_mixed(lu_handle h, cudaStream_t s, const double* rest_src, int64_t re
     // The rest of update k runs on the SMs the panel leaves free; once the
     // panel is done, a helper launch on its stream takes the remaining
     // tiles from the same counter, so the reserved SMs do not idle.
-    unsigned* ctr =
-        (rest > nw && h->gemm_helper && h->gemm_ctas > 0 && h->gemm_reserve > 0) ? h->take_counter() : nullptr;
+    const int reserve = panel_reserve(h->gemm_reserve, h->gemm_ctas, rest);
+    unsigned* ctr = (rest > nw && h->gemm_helper && h->gemm_ctas > 0 && reserve > 0) ? h->take_counter() : nullptr;
     if (ctr)
       LUB_TRY(lowp_gemm(h, mapL, mapU, mapC, k1, rest, nw, rest - nw, K, kpart, kw, bf16, h->sP, 0, ctr,
-                        h->gemm_reserve));
+                        reserve));
     LUB_CUDA(cudaEventRecord(h->evP, h->sP));
     if (rest > nw)
-      LUB_TRY(lowp_gemm(h, mapL, mapU, mapC, k1, rest, nw, rest - nw, K, kpart, kw, bf16, s, h->gemm_reserve,
-                        ctr));
+      LUB_TRY(lowp_gemm(h, mapL, mapU, mapC, k1, rest, nw, rest - nw, K, kpart, kw, bf16, s, reserve, ctr));
   }
   return LU_OK;
 }
@@ -1183,4 +1193,9 @@ extern "C" int lu_refine_solve_host(lu_handle h, const double* hA, int64_t lda, 
   if (pa.type == cudaMemoryTypeDevice || pa.type == cudaMemoryTypeManaged) return LU_ERR_ARG;  // lu_refine_solve
   LUB_TRY(ensure_kernels_init());
   return refine_solve(h, ASrc{hA, lda, true}, db, dx, info, (cudaStream_t)stream);
+}
+
+// Test hook (no GPU): SMs that the trailing update leaves to a panel of M rows.
+extern "C" __attribute__((visibility("default"))) int lub_test_panel_reserve(int gemm_reserve, int gemm_ctas, int M) {
+  return panel_reserve(gemm_reserve, gemm_ctas, M);
 }

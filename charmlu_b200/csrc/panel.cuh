@@ -665,6 +665,9 @@ int leaf_max_width(int M, int num_sms) {
 }
 
 template <typename T>
+int leaf_min_ctas(int M) { return ceil_div(M, NT * leaf_rows<T, 32>()); }
+
+template <typename T>
 int launch_getf2_leaf(T* P, int64_t lda, int M, int ncols, int32_t* ipiv, int row_base, ulonglong2* pkt,
                       unsigned tag0, DevStatus* st, int info_base, double thr, long long spin, int max_ctas,
                       bool alone, cudaStream_t s, T* prow0, int pw, int lc0) {
@@ -699,6 +702,7 @@ int launch_getf2_leaf(T* P, int64_t lda, int M, int ncols, int32_t* ipiv, int ro
 }
 
 #define LUB_INSTANTIATE_LEAF(T)                                                                                    \
+  template int leaf_min_ctas<T>(int);                                                                             \
   template int leaf_max_width<T>(int, int);                                                                       \
   template int launch_getf2_leaf<T>(T*, int64_t, int, int, int32_t*, int, ulonglong2*, unsigned, DevStatus*, int, \
                                     double, long long, int, bool, cudaStream_t, T*, int, int);

@@ -45,3 +45,17 @@ def test_every_promised_leaf_has_a_launch(esize, rows32, rows16, sms, cluster):
                     assert (G - 1) * R < M  # no CTA without rows
                 assert rpt <= {32: rows32, 16: rows16, 8: 12}[W]
                 assert transport == (0 if M <= 2 * NT else 2 if cluster and M <= cluster * NT * rpt else 1)
+
+
+def test_the_update_leaves_a_panel_beside_it_enough_sms():
+    """Under look-ahead the FP32 leaf's cooperative grid fits the SMs that the update
+    does not hold, at every height."""
+    from charmlu_b200 import _lib
+    L = _lib.load()
+    out = np.zeros(7, dtype=np.int32)
+    for M in [16385, 65536, 73728, 73729, 80000, 82000, 90000, 120000, 148 * 6 * NT]:
+        reserve = L.lub_test_panel_reserve(48, 148, M)
+        L.lub_test_leaf_plan(4, M, 32, 148, 48, 0, ctypes.c_void_p(out.ctypes.data))
+        assert out[1] == 0 and out[4] <= reserve <= 148, M
+        assert reserve == 48 or M > 73728
+    assert L.lub_test_panel_reserve(0, 148, 90000) == 0  # no SMs kept on request
