@@ -21,7 +21,7 @@ from ._lib import (LU_ERR_ARG, LU_ERR_NOCONV, LU_ERR_TIMEOUT, LU_ERR_UNSUPPORTED
 
 __all__ = ["LUConfig", "LUSolver", "LUError", "generate_uniform", "matgen", "status_string",
            "LU_PREC_FP64", "LU_PREC_BF16", "LU_PREC_FP16S", "LU_PREC_FP16X3", "LU_PREC_FP32", "LU_IR_CLASSIC", "LU_IR_GMRES",
-           "LU_LAYOUT_ROW", "LU_LAYOUT_COL", "transpose_square"]
+           "LU_LAYOUT_ROW", "LU_LAYOUT_COL", "transpose_square", "pool_release"]
 
 EPS = 2.220446049250313e-16
 
@@ -320,6 +320,12 @@ class LUSolver:
 def launch_count():
     """Kernels liblu_b200 has launched since it was loaded."""
     return int(_lib.load().lu_launch_count())
+
+
+def pool_release():
+    """Free the device memory that closed solvers left for later ones on the
+    current device (lu_pool_release)."""
+    _check(_lib.load().lu_pool_release(), "lu_pool_release")
 
 
 def transpose_square(A, stream=None):

@@ -25,7 +25,7 @@ EXPORTS = [
     "lu_batched_work_bytes", "lu_batched_set_tuning", "lu_refine_factor", "lu_refine_apply",
     "lu_refine_adjoint", "lu_panel_factor", "lu_apply_pivots", "lu_trsm_lower_unit", "lu_gemm_update",
     "lu_trsv_block", "lu_gemv_update", "lu_copy_2d", "lu_transpose_square", "lu_status_clear",
-    "lu_refine_precond_norm", "lu_batched_refine_histogram",
+    "lu_refine_precond_norm", "lu_batched_refine_histogram", "lu_pool_release",
 ]
 PHASES = ["panel", "laswp", "trsm", "gemm", "gemm_inner", "solve", "other"]
 
@@ -68,6 +68,7 @@ def load():
         "lu_config_default": ([ctypes.POINTER(LuConfig), i64, i32], ctypes.c_int),
         "lu_create": ([ctypes.POINTER(LuConfig), ctypes.POINTER(H)], ctypes.c_int),
         "lu_destroy": ([H], ctypes.c_int),
+        "lu_pool_release": ([], ctypes.c_int),
         "lu_workspace_bytes": ([ctypes.POINTER(LuConfig)], ctypes.c_size_t),
         "lu_status": ([H, P], ctypes.c_int),
         "lu_factor": ([H, P, i64, P, P, P], ctypes.c_int),

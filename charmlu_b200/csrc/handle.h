@@ -35,8 +35,9 @@ int ensure_kernels_init();
 // blocks, and streams, events and a pinned word.  A program that makes a handle
 // per call (autograd does) otherwise spends 2 - 11 ms in some twenty
 // allocations and frees, each of which may wait for the device.  Bounded (1/64
-// of the device's memory, 8 sets of streams), given back when an allocation
-// fails or after 32 destroys without use; every function locks.
+// of the device's memory or LU_B200_POOL_BYTES if that is less, 8 sets of
+// streams), given back by lu_pool_release, when an allocation fails or after 32
+// destroys without use; every function locks.
 struct HandleRes {
   cudaStream_t sP = nullptr, sG = nullptr;  // sP: highest priority
   cudaEvent_t ev[6] = {};                   // timing disabled
@@ -45,10 +46,13 @@ struct HandleRes {
 int pool_alloc(void** p, size_t bytes, size_t* got);
 // a new block of the caller's own, for cudaFree
 int pool_malloc(void** p, size_t bytes);
-// p must not be in use by the device any more
-void pool_free(int device, void* p, size_t bytes);
+// p must not be in use by the device any more; limit: bytes that the pool may
+// hold (0: nothing is kept)
+void pool_free(int device, void* p, size_t bytes, size_t limit);
 int pool_take_res(HandleRes* r);
-void pool_give_res(int device, const HandleRes& r);
+void pool_give_res(int device, const HandleRes& r, size_t limit);
+// frees what the current device's pool holds
+int pool_release();
 
 }  // namespace lub
 
@@ -177,6 +181,7 @@ struct lu_handle_s {
   int64_t res_elems = 0;
   int res_rows = 0;
   size_t resident_cap = ~size_t(0);
+  size_t pool_limit = ~size_t(0);  // LU_B200_POOL_BYTES
   int64_t host_copied = 0;  // bytes of host A copied to the device, running total
   std::vector<std::pair<void*, size_t>> allocs;  // block, its size in the pool
   lub::HandleRes res;

@@ -361,6 +361,7 @@ int lu_create(const lu_config* cfg, lu_handle* out) {
   if (const char* e = getenv("LU_B200_TRSM_WIDE")) h->trsm_wide = atoi(e) != 0;
   if (const char* e = getenv("LU_B200_TRSM_WIDE_MIN")) h->trsm_wide_min = std::max(0, atoi(e));
   if (const char* e = getenv("LU_B200_STAGE_BYTES")) h->stage_bytes = std::max<size_t>(1 << 16, strtoull(e, nullptr, 10));
+  if (const char* e = getenv("LU_B200_POOL_BYTES")) h->pool_limit = strtoull(e, nullptr, 10);
   if (const char* e = getenv("LU_B200_RESIDENT_BYTES")) h->resident_cap = strtoull(e, nullptr, 10);
   if (s == LU_OK) s = h->alloc(&h->perm, n);
   if (s == LU_OK) s = h->alloc(&h->perm_work, n);
@@ -399,17 +400,18 @@ int lu_destroy(lu_handle h) {
   const bool idle = cudaFree(h->st) == cudaSuccess;
   if (!idle) cudaGetLastError();
   for (auto& blk : h->allocs) {
-    if (idle) pool_free(h->device, blk.first, blk.second);
+    if (idle) pool_free(h->device, blk.first, blk.second, h->pool_limit);
     else cudaFree(blk.first);
   }
   if (h->res.sP) {
-    if (idle) pool_give_res(h->device, h->res);
-    else pool_give_res(-1, h->res);
+    pool_give_res(idle ? h->device : -1, h->res, h->pool_limit);
   }
   if (cur != h->device) cudaSetDevice(cur);
   delete h;
   return LU_OK;
 }
+
+int lu_pool_release(void) { return pool_release(); }
 
 int lu_status(lu_handle h, void* stream) {
   if (!h) return LU_ERR_ARG;

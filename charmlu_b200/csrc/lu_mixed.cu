@@ -528,6 +528,7 @@ int ensure_staging(lu_handle h, int64_t lda) {
 // current copy counts as free, since it is replaced. Sets h->res_rows.
 int ensure_resident(lu_handle h, int64_t lda, int n) {
   size_t free_b = 0, total_b = 0;
+  pool_release();  // what destroyed handles left counts as free
   LUB_CUDA(cudaMemGetInfo(&free_b, &total_b));
   const size_t have = (size_t)h->res_elems * sizeof(double);
   const size_t margin = std::max<size_t>(size_t(2) << 30, total_b / 32);

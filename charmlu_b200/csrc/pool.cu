@@ -100,7 +100,7 @@ int pool_malloc(void** p, size_t bytes) {
   return malloc_or_empty(d, p, bytes);
 }
 
-void pool_free(int device, void* p, size_t bytes) {
+void pool_free(int device, void* p, size_t bytes, size_t limit) {
   if (device < 0 || device >= 64) {
     cudaFree(p);
     return;
@@ -109,15 +109,26 @@ void pool_free(int device, void* p, size_t bytes) {
   std::lock_guard<std::mutex> lk(d.mu);
   if (!d.cap) {
     size_t fr = 0, total = 0;
-    if (cudaMemGetInfo(&fr, &total) != cudaSuccess) cudaGetLastError();
-    d.cap = total / 64 + 1;
+    if (cudaMemGetInfo(&fr, &total) == cudaSuccess) d.cap = total / 64;
+    else cudaGetLastError();
   }
-  if (d.cached + bytes > d.cap) {
+  if (d.cached + bytes > std::min(limit, d.cap)) {
     cudaFree(p);
     return;
   }
   d.blocks.push_back({p, bytes, d.tick});
   d.cached += bytes;
+}
+
+int pool_release() {
+  int dev = 0;
+  LUB_TRY(current_device(&dev));
+  DevPool& d = pool_of(dev);
+  std::lock_guard<std::mutex> lk(d.mu);
+  for (size_t i = d.blocks.size(); i-- > 0;) drop(d, i);
+  for (const HandleRes& r : d.res) destroy_res(r);
+  d.res.clear();
+  return d.blocks.empty() ? LU_OK : LU_ERR_CUDA;
 }
 
 int pool_take_res(HandleRes* r) {
@@ -144,7 +155,7 @@ int pool_take_res(HandleRes* r) {
   return LU_ERR_CUDA;
 }
 
-void pool_give_res(int device, const HandleRes& r) {
+void pool_give_res(int device, const HandleRes& r, size_t limit) {
   if (device < 0 || device >= 64) {
     destroy_res(r);
     return;
@@ -154,8 +165,8 @@ void pool_give_res(int device, const HandleRes& r) {
   // once per destroy: blocks that nothing has asked for since long go back
   d.tick++;
   for (size_t i = d.blocks.size(); i-- > 0;)
-    if (d.tick - d.blocks[i].tick > kIdleDestroys) drop(d, i);
-  if (d.res.size() < kMaxRes) d.res.push_back(r);
+    if (d.tick - d.blocks[i].tick > kIdleDestroys || d.cached > limit) drop(d, i);
+  if (limit > 0 && d.res.size() < kMaxRes) d.res.push_back(r);
   else destroy_res(r);
 }
 

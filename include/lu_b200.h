@@ -130,11 +130,16 @@ typedef struct lu_refine_info {
 LU_API int lu_config_default(lu_config* cfg, int64_t n, int32_t block_size);
 
 /* Create / destroy a solver handle on the current device; allocates the
- * handle's workspace (candidate slots, barrier counters, pivot lists).
+ * handle's workspace (candidate packets, counters, pivot lists).
  * Replaces LUSolver construction + LUBlk::startup (benchmark.C:258-294,
- * lu.ci:467-494). */
+ * lu.ci:467-494).  lu_destroy waits for the device's work.  It leaves the
+ * handle's memory to handles made later: at most 1/64 of the device's memory, or
+ * LU_B200_POOL_BYTES as it was at lu_create if that is less (0: nothing). */
 LU_API int lu_create(const lu_config* cfg, lu_handle* out);
 LU_API int lu_destroy(lu_handle h);
+/* Free what destroyed handles left on the current device, for other users of its
+ * memory.  Handles in use are not affected. */
+LU_API int lu_pool_release(void);
 /* Device workspace bytes the handle holds (precision-dependent). */
 LU_API size_t lu_workspace_bytes(const lu_config* cfg);
 

@@ -245,3 +245,31 @@ def test_handles_are_not_made_inside_a_capture(cuda_dev, pooled):
     lu.LUSolver(lu.LUConfig(n, 64)).close()
     kept.close()
     first.close()
+
+
+def test_pool_memory_goes_back(cuda_dev, monkeypatch):
+    """lu_pool_release frees what closed solvers left; a bound of 0 leaves nothing."""
+    import charmlu_b200 as lu
+    n = 4096
+    A = lu.generate_uniform(n, n, seed=1)
+    A.diagonal().add_(float(n) ** 0.5)
+    b = lu.generate_uniform(n, 1, seed=2).view(-1)
+
+    def use():
+        s = lu.LUSolver(lu.LUConfig(n, 128, precision=lu.LU_PREC_FP16X3))
+        x, info = s.refine_solve(A, b)
+        assert info["status"] == 0
+        s.close()
+        return torch.cuda.mem_get_info()[0]
+
+    use()  # kernels loaded, torch's own blocks in place
+    lu.pool_release()
+    free = torch.cuda.mem_get_info()[0]
+    assert use() <= free - 4 * n * n  # the FP32 factors alone
+    lu.pool_release()
+    assert torch.cuda.mem_get_info()[0] == free
+    monkeypatch.setenv("LU_B200_POOL_BYTES", "0")
+    assert use() == free
+    monkeypatch.setenv("LU_B200_POOL_BYTES", str(1 << 20))
+    assert use() >= free - (4 << 20)
+    lu.pool_release()
