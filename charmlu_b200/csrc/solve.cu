@@ -982,8 +982,12 @@ int launch_trsv_mixed(const TS* LU, int64_t lda, int n, T* x, int upper, int* fl
           cudaFuncSetAttribute(trsv_kernel<TS, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return r;
   }));
-  // flags[0] is the progress counter, flags[1] the ticket that hands out block order
-  LUB_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * kTrsvScratchInts, s));
+  // flags[0] is the progress counter, flags[1] the ticket that hands out block
+  // order; then the ring's slots, of which as many are read as there are blocks
+  // ahead of the last one.  A clear of more than 2 KB costs the host 5 us, one of
+  // 32 bytes 1.7 (one block: 26 us a call with the whole ring cleared, 21 without)
+  const int slots = std::min(nblk - 1, kPipeRing);
+  LUB_CUDA(cudaMemsetAsync(flags, 0, sizeof(int) * (8 + slots * TB * 4), s));
   if (upper)
     trsv_kernel<TS, T, true><<<nblk, 256, smem, s>>>(LU, lda, n, x, flags, st, spin);
   else

@@ -48,3 +48,23 @@ def test_repeated_solves_give_the_same_bits(cuda_dev, nrhs):
         scale = A.abs().sum(1).max() * first.abs().max() + B.abs().max()
         assert R.abs().max() < 16 * n * 2.0 ** -52 * scale
     s.close()
+
+
+@pytest.mark.parametrize("upper", [0, 1])
+def test_substitutions_of_changing_size_share_one_ring(cuda_dev, upper):
+    """Orders of 1 to 6 blocks in turn through one handle: the ring of packets
+    starts cleared as far as a call reads it, whatever the call before left."""
+    from charmlu_b200.blocks import CudaBlocks
+    bl = CudaBlocks(384, 64)
+    gen = torch.Generator(device="cuda").manual_seed(upper)
+    for it in range(4):
+        for w in [384, 64, 320, 65, 256, 128, 257, 129, 1, 192, 384, 193, 2]:
+            T = torch.zeros(w, w + (w & 1), dtype=torch.float64, device="cuda")[:, :w]
+            T.copy_((torch.rand(w, w, dtype=torch.float64, device="cuda", generator=gen) - 0.5) * 0.1)
+            T.diagonal().fill_(1.0)
+            x = torch.rand(w, dtype=torch.float64, device="cuda", generator=gen)
+            ref = torch.linalg.solve_triangular(T, x.view(-1, 1), upper=bool(upper), unitriangular=not upper).view(-1)
+            bl.trsv_block(T, upper, x)
+            # |T| <= 1 off a unit diagonal of small rows: both are within w roundings of the size
+            assert (x - ref).abs().max() <= 1e-12 * ref.abs().max(), (it, w)
+    bl.close()
