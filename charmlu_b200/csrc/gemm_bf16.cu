@@ -776,8 +776,11 @@ gemm_lowp_pair_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
         }
         fence_proxy_async();
         epi_bar();
-        if (leader && rows_in) {
-          tma_reduce_add_2d(&mapC, box, args.c_col0 + tn * BN + c * EPI_COLS, crow);
+        // a group per chunk even where there is nothing to add: the wait for
+        // the box of two chunks ago counts groups, so without it a tile below
+        // M would write over the last box of the tile before while it is read
+        if (leader) {
+          if (rows_in) tma_reduce_add_2d(&mapC, box, args.c_col0 + tn * BN + c * EPI_COLS, crow);
           bulk_commit();
         }
       }

@@ -704,3 +704,28 @@ def test_refine_wide_u_solve(cuda_dev, n, b, la, monkeypatch):
         assert s.residual(A, x, rhs)["r_hpl"] < 16
         fe = np.abs(x.cpu().numpy() - x_ref).max() / np.abs(x_ref).max()
         assert fe < 1e-6, fe
+
+
+@pytest.mark.parametrize("M", [296, 384, 1064])
+@pytest.mark.parametrize("ctas", [2, 8])
+def test_pair_update_with_half_a_tile_row_below_the_matrix(cuda_dev, M, ctas):
+    """The odd CTA of a pair has nothing to add for a last tile row of 1 to 128 rows.
+    Its tiles before and after that keep their values: the same bits as one CTA
+    per tile row, in every repetition."""
+    f = _lib()
+    K, N = 64, 8192
+    g = torch.Generator(device="cuda").manual_seed(M)
+    A = torch.rand(M, K, device="cuda", generator=g) - 0.5
+    B = torch.rand(K, N, device="cuda", generator=g) - 0.5
+    C0 = torch.rand(M, N, device="cuda", generator=g) - 0.5
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def run(mode):
+        C = C0.clone()
+        assert f(A.data_ptr(), K, B.data_ptr(), N, C.data_ptr(), N, M, N, K, mode, stream) == 0
+        return C
+
+    want = run(3 | 32 << 8)  # tiles of one CTA
+    for _ in range(25):
+        assert torch.equal(run(3 | ctas << 8 | 1 << 24), want)
+        assert torch.equal(run(3 | ctas << 8 | 4 << 16 | 1 << 24), want)  # with a second launch on another stream
