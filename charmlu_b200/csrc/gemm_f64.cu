@@ -69,7 +69,7 @@ gemm_f64_sub_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_const
   if (tid == 0) {
     // the first CTA in an SM's second slot starts about half a tile later:
     // without that both CTAs of an SM load and store C at the same times
-    if (gridDim.x >= 8 * kNumSMsB200 && blockIdx.x < 2 * kNumSMsB200) {
+    if (args.stagger && blockIdx.x < 2 * kNumSMsB200) {
       unsigned w;
       asm volatile("mov.u32 %0, %%warpid;" : "=r"(w));
       if ((w / (THREADS / 32)) & 1)
@@ -236,7 +236,16 @@ int launch_gemm_f64_sub(const CUtensorMap& mapA, const CUtensorMap& mapB, const 
     return LU_ERR_ALIGN;
   const int64_t tiles = (int64_t)ceil_div(a.N, BN) * ceil_div(a.M, BM);
   if (tiles > INT32_MAX) return LU_ERR_UNSUPPORTED;
-  return launch_dependent(gemm_f64_sub_kernel, dim3((unsigned)tiles), dim3(THREADS), SMEM_BYTES, stream, mapA, mapB, a);
+  // The late start costs nothing where the last round is at most half full (3.5
+  // rounds, 32768 x 256, K = 128: 77 us with it, 92 without).  Otherwise it costs
+  // half a tile at the end, and what it saves on C is the same per round at any
+  // K: it pays from K / 72 rounds on (3328 x 3328, 4.6 rounds, K = 256 201 / 207
+  // us, K = 1024 750 / 727; 8192 x 8192, 28 rounds, K = 2048 7.95 / 7.92 ms).
+  constexpr int64_t slots = 2 * kNumSMsB200;
+  const int64_t last = tiles % slots;
+  GemmArgs b = a;
+  b.stagger = last > 0 && 2 * last <= slots ? tiles >= 3 * slots : tiles >= 4 * slots && 72 * tiles >= a.K * slots;
+  return launch_dependent(gemm_f64_sub_kernel, dim3((unsigned)tiles), dim3(THREADS), SMEM_BYTES, stream, mapA, mapB, b);
 }
 
 }  // namespace lub

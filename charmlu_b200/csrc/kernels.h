@@ -13,6 +13,7 @@ struct GemmArgs {
   int M, N, K;
   DevStatus* st;
   long long spin;
+  int stagger = 0;  // set by the launch: the second CTA of an SM starts late
 };
 int gemm_f64_init();
 int gemm_f64_smem_bytes();

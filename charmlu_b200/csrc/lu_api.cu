@@ -110,16 +110,24 @@ int pivots_apply_f64(Ctx64& c, int k0, int cnt, int c_begin, int c_end, int skip
   return LU_OK;
 }
 
+// Products in 64 x 32 tiles: those of up to 64 columns (n = 2048, b = 128: 5.01 ->
+// 4.68 ms; n = 16384 135.4 -> 132.0), and those of at most two rounds of 128 x 64
+// tiles on two slots per SM where the rounds are not filled: a round takes as long
+// as 960 to 1030 small tiles, the fewer the larger K is, however few tiles are
+// in it.  B200, 64 x 32 / 128 x 64 tiles, K = 256: 1280 x 1280 35.9 / 39.6 us, 1536 x 1536 46.6 /
+// 40.1, 1792 x 1792 62.6 / 78.2, 2176 x 2176 88.9 / 79.1.  The same bits.
+bool gemm64_small(int M, int N, int K) {
+  if (N <= 64) return true;
+  const int64_t small = (int64_t)ceil_div(M, 64) * ceil_div(N, 32), large = (int64_t)ceil_div(M, 128) * ceil_div(N, 64);
+  const int64_t rounds = (large + 2 * kNumSMsB200 - 1) / (2 * kNumSMsB200);
+  return rounds <= 2 && small <= rounds * (K < 256 ? 1030 : K < 512 ? 1000 : 960);
+}
+
 // C(rc, cc) [M x N] -= A(ra, ca) [M x K] * B(rb, cb) [K x N]
 int gemm64(Ctx64& c, const MatF64& Cm, int rc, int cc, const MatF64& Am, int ra, int ca, const MatF64& Bm, int rb,
            int cb, int M, int N, int K, int phase = LU_PH_GEMM_IN) {
   Prof pf(c.h, c.s, phase, 2.0 * M * (double)N * K);
-  // 64 x 32 tiles where half or more of a 128-wide tile's columns would be
-  // padding (n = 2048, b = 128: 5.01 -> 4.68 ms; n = 16384 135.4 -> 132.0) or
-  // where 128 x 128 tiles make fewer than two waves (2048: 4.68 -> 4.54; 16384:
-  // 132.0 -> 131.1); the same bits
-  const int64_t tiles = (int64_t)ceil_div(M, 128) * ceil_div(N, 128);
-  if (N <= 64 || tiles <= 2 * kNumSMsB200) {
+  if (gemm64_small(M, N, K)) {
     if ((ca & 1) || (cb & 1) || (cc & 1)) return LU_ERR_ALIGN;
     return launch_gemm_f64_small(Am.at(ra, ca), Am.ld, Bm.at(rb, cb), Bm.ld, Cm.at(rc, cc), Cm.ld, M, N, K, c.s);
   }

@@ -63,3 +63,26 @@ def test_one_launch_solve_gives_the_recursions_bits(cuda_dev, w, ncols):
     out.copy_(B)
     bl.trsm_lower_unit(L, out)
     assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("M,N,K", [(1280, 1280, 130), (1536, 1408, 64), (1536, 1536, 257), (1792, 1800, 255),
+                                   (2048, 2048, 192), (2048, 2048, 300), (2177, 2175, 96), (2304, 2304, 40),
+                                   (3328, 3328, 33), (3328, 3328, 1030)])
+def test_every_choice_of_tiles_gives_the_same_bits(cuda_dev, M, N, K):
+    """Products on both sides of the lines between small and large tiles, and with
+    and without the late start of an SM's second CTA, against slices of 64 columns."""
+    from charmlu_b200.blocks import CudaBlocks
+    bl = CudaBlocks(4096, 64)
+    gen = torch.Generator(device="cuda").manual_seed(M + K)
+
+    def mat(r, c):
+        return torch.rand(r, c + (c & 1), dtype=torch.float64, device="cuda", generator=gen)[:, :c].sub_(0.5)
+
+    A, B, C = mat(M, K), mat(K, N), mat(M, N)
+    D = torch.empty(M, N + (N & 1), dtype=torch.float64, device="cuda")[:, :N]
+    D.copy_(C)
+    bl.gemm_update(A, B, C)
+    for c in range(0, N, 64):
+        bl.gemm_update(A, B[:, c:c + 64], D[:, c:c + 64])
+    assert torch.equal(C, D)
+    bl.close()
