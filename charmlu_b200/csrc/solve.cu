@@ -397,10 +397,11 @@ __device__ __forceinline__ bool wait_progress(const int* counter, int need, int*
 // backwards, and who acquires tk + 2 could read block tk's rows before they are
 // there; in turn, every store of the counter follows the rows of all blocks up
 // to its value.  The packets have left by now, so this is not on the chain.
-// Called by one thread; bounded as wait_progress.
+// Called by one thread, not for the last block, which nobody waits for; bounded as
+// wait_progress.
 __device__ __forceinline__ void publish_progress(int* counter, int tk, DevStatus* st, long long spin, int where) {
   int v;
-  if (wait_progress(counter, tk, &v, st, spin, where)) st_release_s32(counter, tk + 1);
+  if (tk == 0 || wait_progress(counter, tk, &v, st, spin, where)) st_release_s32(counter, tk + 1);
 }
 
 // A finished block's rows also leave as 16-byte packets {value, tag} in a ring
@@ -589,7 +590,7 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TS* LU, int64_t lda, in
   // CTA barrier, then thread 0's release store: the rows written above are
   // visible to every CTA that acquires the counter
   __syncthreads();
-  if (tid == 0) publish_progress(&flags[0], tk, st, spin, 301);
+  if (tid == 0 && tk + 1 < nblk) publish_progress(&flags[0], tk, st, spin, 301);
 }
 
 // ---------------------------------------------------------------------------
@@ -809,7 +810,7 @@ __global__ void __launch_bounds__(256, 2) trsm_pipe_kernel(const TS* LU, int64_t
   // CTA barrier, then thread 0's release store: the rows written above are
   // visible to every CTA that acquires the counter
   __syncthreads();
-  if (tid == 0) publish_progress(progress, tk, st, spin, 302);
+  if (tid == 0 && tk + 1 < nblk) publish_progress(progress, tk, st, spin, 302);
 }
 
 // G = -Lam * X^T (n x n), Lam and X n x k row-major, k <= 16: the rank-k
