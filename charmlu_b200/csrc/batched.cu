@@ -73,7 +73,7 @@ struct WorkHeader {
   unsigned queue;
   int bad;          // nonzero: an order outside [1, kBatchMaxN] or workspace too small
   long long s1, s2; // sum n, sum n^2
-  long long order, offA32, offV, piv, A32, r64, v32, total;
+  long long order, offA32, offV, A32, r64, total;
   // FP32 mode: systems that reached r_hpl < 16 after s FP64 refinement
   // steps (s = 0 .. 10), and in the last bin those that did not
   int refine_hist[kRefineHistBins];
@@ -1298,14 +1298,10 @@ __global__ void __launch_bounds__(1024) batched_prep_kernel(int count, const int
     hdr->offA32 = o_offA32;
     hdr->offV = o_offV;
     long long q = o;
-    hdr->piv = q;
-    q = align256(q + 4 * s1);
     hdr->A32 = q;
     if (precision == LU_PREC_FP32) q = align256(q + 4 * s2);
     hdr->r64 = q;
     if (precision == LU_PREC_FP32) q = align256(q + 16 * s1);
-    hdr->v32 = q;
-    if (precision == LU_PREC_FP32) q = align256(q + 4 * s1);
     hdr->total = q;
     if (q > work_bytes) s_bad = 1;
   }
@@ -1342,11 +1338,9 @@ extern "C" LU_API size_t lu_batched_work_bytes(int32_t count, const int32_t* n_h
   o = align256(o + 4LL * count);
   o = align256(o + 8LL * count);
   o = align256(o + 8LL * count);
-  o = align256(o + 4 * s1);
   if (precision == LU_PREC_FP32) {
     o = align256(o + 4 * s2);
     o = align256(o + 16 * s1);
-    o = align256(o + 4 * s1);
   }
   return (size_t)o;
 }

@@ -170,43 +170,13 @@ __device__ __forceinline__ void dev_singular(DevStatus* st, int col1) {
   }
 }
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ int ld_acquire_s32(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void red_release_add_u32(unsigned* p, unsigned v) {
-  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ void st_release_s32(int* p, int v) {
   asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Grid-wide barrier on a dedicated counter (zeroed before the launch): the
-// n-th call waits until the counter reaches n * nblocks.  Bounded: returns
-// false after spin_limit polls (status set), or when another block already
-// failed.
-__device__ __forceinline__ bool grid_barrier(unsigned* counter, unsigned target, DevStatus* st,
-                                             long long spin_limit, int where) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    red_release_add_u32(counter, 1u);
-    long long polls = 0;
-    while (ld_acquire_u32(counter) < target) {
-      if (++polls > spin_limit) { dev_fail(st, LU_ERR_TIMEOUT, where); ok = 0; break; }
-      if ((polls & 255) == 0 && ld_acquire_s32(&st->code) != 0) { ok = 0; break; }
-    }
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
 }
 
 // Grouped raster over an ntm x ntn tile grid: blocks run down groups of

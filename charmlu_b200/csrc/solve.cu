@@ -406,9 +406,9 @@ __device__ __forceinline__ void publish_progress(int* counter, int tk, DevStatus
 
 // A finished block's rows also leave as 16-byte packets {value, tag} in a ring
 // of kPipeRing blocks, ahead of the counter (n = 8192, forward and backward:
-// one column 864 -> 608 us; 16 columns, with two chains, 840 -> 739 us): one 128-bit access each, so the
-// data is its own flag, and the next blocks read them without the publisher's
-// fence and a second trip for the rows.  A block takes its last
+// one column 864 -> 608 us; 16 columns, with two chains, 840 -> 739 us): one
+// 128-bit access each, so the data is its own flag, and the next blocks read
+// them without the publisher's fence and a second trip for the rows.  A block takes its last
 // kPipeRing - 1 predecessors this way; that the ring's slot of block t - 4 is
 // free when block t publishes follows from t having waited for t - 1, which
 // had waited for t - 2 and t - 3: the only readers of that slot.
@@ -608,10 +608,10 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TS* LU, int64_t lda, in
 // against the finished rows of Y, and the inverted diagonal tile against the
 // block's right-hand side) run on the FP64 tensor pipe (mma.sync m16n8k4; warp
 // w < 4 owns output rows 16 w ..).  With 16 columns in one chain each product
-// kept two warps of an SM sub-partition waiting for the pipe in turn.  The factor tiles do not depend on the pipeline, so they
-// stream through a two-stage cp.async ring (tile q+1 in flight while the
-// CTA waits for block q and applies tile q); only the 64 x 16 slice of Y
-// waits for the counter.  Tiles are read by rows in every mode (the
+// kept two warps of an SM sub-partition waiting for the pipe in turn.  The
+// factor tiles do not depend on the pipeline, so they stream through a
+// two-stage cp.async ring (tile q+1 in flight while the CTA waits for block q
+// and applies tile q); only the 64 x 8 slice of Y waits for packets or counter.  Tiles are read by rows in every mode (the
 // transposed modes index the staged tile transposed).  Pitches keep the
 // fragment loads free of bank conflicts.
 // Dynamic shared memory: the ring, then the FP64 inverse of the diagonal

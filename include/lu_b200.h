@@ -258,7 +258,7 @@ LU_API int lu_adjoint(lu_handle h, const double* dLU, int64_t lda, const int32_t
 
 /* Batched factor+solve of many independent systems of uneven order in one
  * persistent launch (no reference counterpart).  System i has order n[i]
- * (1 <= n[i] <= 1536), its matrix at dA + a_off[i] (row-major, lda = n[i])
+ * (1 <= n[i] <= 2048), its matrix at dA + a_off[i] (row-major, lda = n[i])
  * and right-hand side at db + b_off[i] (overwritten by x).  precision:
  *   LU_PREC_FP64  FP64 factors in place in dA (as lu_factor);
  *   LU_PREC_FP32  FP32 factors of a copy in dWork, then FP64 refinement
