@@ -406,7 +406,7 @@ __device__ __forceinline__ void publish_progress(int* counter, int tk, DevStatus
 
 // A finished block's rows also leave as 16-byte packets {value, tag} in a ring
 // of kPipeRing blocks, ahead of the counter (n = 8192, forward and backward:
-// one column 864 -> 608 us; 16 columns, with two chains, 840 -> 739 us): one
+// one column 864 -> 608 us; 16 columns, with two chains, 843 -> 747 us): one
 // 128-bit access each, so the data is its own flag, and the next blocks read
 // them without the publisher's fence and a second trip for the rows.  A block takes its last
 // kPipeRing - 1 predecessors this way; that the ring's slot of block t - 4 is

@@ -138,7 +138,8 @@ LU_API int lu_config_default(lu_config* cfg, int64_t n, int32_t block_size);
 LU_API int lu_create(const lu_config* cfg, lu_handle* out);
 LU_API int lu_destroy(lu_handle h);
 /* Free what destroyed handles left on the current device, for other users of its
- * memory.  Handles in use are not affected. */
+ * memory.  Handles in use are not affected.  LU_ERR_CUDA if something could not
+ * be freed (while the thread captures, for one). */
 LU_API int lu_pool_release(void);
 /* Device workspace bytes the handle holds (precision-dependent). */
 LU_API size_t lu_workspace_bytes(const lu_config* cfg);
